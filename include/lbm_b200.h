@@ -276,7 +276,9 @@ int lbm_init_equilibrium(lbm_solver *s, unsigned long long seed, double amplitud
 /* Free and total memory of the current CUDA device (cudaMemGetInfo). */
 int lbm_device_memory(size_t *free_bytes, size_t *total_bytes);
 
-/* Enqueues `steps` time steps on the solver's stream (asynchronous).
+/* Enqueues `steps` time steps on the solver's stream (asynchronous). Several
+ * steps may run in one launch; the states are those of single steps, bit for
+ * bit.
  * Replaces the time loop of kd->Kernel (src/kernel_pull_soa.c:44-214,
  * src/kernel_push_soa.c:44-214, src/kernel_aa_soa.c:36-286); an AA solver
  * runs single steps, so odd counts are allowed. */
@@ -382,7 +384,8 @@ long long lbm_steps_done(const lbm_solver *s);
 size_t lbm_device_bytes(const lbm_solver *s);
 /* Algorithmic bytes moved per fluid lattice update: 2 * 19 * storage size. */
 double lbm_bytes_per_update(const lbm_solver *s);
-/* Number of step-kernel launches issued since creation. */
+/* Number of step-kernel launches issued since creation (one launch of lbm_run
+ * may take several steps). */
 long long lbm_launch_count(const lbm_solver *s);
 
 const char *lbm_last_error(void);

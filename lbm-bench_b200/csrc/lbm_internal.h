@@ -10,6 +10,7 @@
 #include "lbm_step.cuh"
 #include "lbm_step_cp.cuh"
 #include "lbm_step_tma.cuh"
+#include "lbm_sweep.cuh"
 #include "lbm_step_x2.cuh"
 
 namespace lbm {
@@ -38,6 +39,20 @@ cudaError_t launch_step_cp_f64(int kind, bool force, const StepArgs<StoreF64> &a
 cudaError_t launch_step_cp2_f32(int kind, bool force, const StepArgs2<StoreF32> &a,
     cudaStream_t st);
 cudaError_t launch_step_cp2_f16(int kind, bool force, const StepArgs2<StoreF16> &a,
+    cudaStream_t st);
+
+// Sweeps (lbm_sweep.cuh, lbm_sweep_x2.cuh). `flip`: the pull orientation;
+// plan.lag > 0: fronts, else step-major.
+struct SweepLaunch {
+  Grid g;
+  void *f; // the lattice
+  const uint32_t *mask;
+  const float *porosity; // Brinkman term, or NULL
+  SweepPlan p;
+  bool force, flip;
+};
+cudaError_t launch_sweep_f64(const SweepLaunch &l, const Consts<double> &c, cudaStream_t st);
+cudaError_t launch_sweep_x2(int precision, const SweepLaunch &l, const Consts2 &c,
     cudaStream_t st);
 
 // Zou-He pressure boundary on the state after a step (lbm_step_f64.cu):

@@ -77,7 +77,7 @@ struct lbm_solver {
   int tma;           // FP64 steps use the bulk-copy pipelined kernels (shape in tma_shape)
   int tma_groups;    // consumer groups of 8 warps per CTA
   TmaShape tma_shape;
-  unsigned int *dev_err; // set by kernels whose bounded waits ran out
+  unsigned int *dev_err; // set by kernels whose bounded waits ran out (kErr bits)
   uint8_t *bc_marks;     // [2][ny][nz]: inlet / outlet cells of the pressure boundary, or NULL
   int bc_on;
   double rho_in, rho_out;
@@ -91,6 +91,11 @@ struct lbm_solver {
   int compact;
   uint2 *cwb; // compact layout: (fluid bits, first index) per row word
   std::vector<uint32_t> *cplane0; // storage index of the first fluid cell of each x plane (nx+1)
+  // sweeps (lbm_sweep.cuh): several steps per launch, planned at creation
+  int sweep_steps;      // most steps of one launch; 0: single steps only
+  SweepPlan sweep;
+  uint32_t *sweep_done; // its counters
+  int err_pending;      // a launch that may set dev_err is not yet checked
 };
 
 extern "C" const char *lbm_last_error(void) { return g_err; }
@@ -543,6 +548,7 @@ static void free_all(lbm_solver *s)
   cudaFree(s->bc_marks);
   cudaFree(s->cwb);
   delete s->cplane0;
+  cudaFree(s->sweep_done);
   free(s->split_done);
   if (s->fork_ev)
     cudaEventDestroy(s->fork_ev);
@@ -572,9 +578,76 @@ static int dev_alloc(lbm_solver *s, void **p, size_t bytes, const char *what)
   return LBM_OK;
 }
 
+// Waits for the solver's stream, then reports a kernel whose bounded wait ran
+// out since the last check (the error word is copied only if a launch may
+// have set it).
+static int sync_and_check(lbm_solver *s)
+{
+  unsigned int err = 0;
+  if (s->err_pending)
+    CUDA_TRY(cudaMemcpyAsync(&err, s->dev_err, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  if (!s->err_pending)
+    return LBM_OK;
+  s->err_pending = 0;
+  if (!err)
+    return LBM_OK;
+  CUDA_TRY(cudaMemset(s->dev_err, 0, sizeof(err)));
+  return fail(LBM_ERR_CUDA, "a step kernel gave up waiting for %s; the state is undefined",
+      err & kErrBulkCopy ? "its bulk copies" : "the blocks of an earlier step");
+}
+
 // ---------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------
+
+// Whether, and in which order, a solver runs sweeps, and their plan. The
+// lines (lattice bytes, or cells) are where sweeps stop to win over single
+// steps; us per step, single steps / step-major / fronts, channels of 64 x 64
+// planes on a B200:
+//   compact FP64 AA    43 MB 12.4 / 9.6 / 14.9   65 MB 16.6 / 14.3 / 19.6
+//                      87 MB 25.8 / 24.6 / 24.3   108 MB 39.0 / 37.2 / 29.7
+//   compact FP64 pull  43 MB 14.4 / 9.6 / 14.2   87 MB 33.5 / 24.9 / 24.5
+//   compact FP32 AA    43 MB 14.8 / 11.8 / 17.0   87 MB 28.2 / 26.8 / 29.0
+//                      97 MB 34.4 / 33.7 / 32.1   130 MB 48.7 / 49.4 / 41.6
+//   compact FP16 AA    22 MB 13.4 / 11.7 / 16.9   33 MB 17.5 / 17.4 / 22.6
+//                      43 MB 22.2 / 23.1 / 28.4   97 MB 50.0 / 55.4 / 57.9
+//   compact FP16 pull  43 MB 26.7 / 22.9 / 27.4   97 MB 57.5 / 54.5 / 57.3
+//   dense FP64 AA      43 MB 12.4 / 11.2 / 16.0   65 MB 16.5 / 16.9 / 21.3
+//                      87 MB 23.6 / 25.9 / 27.5   108 MB 35.8 / 37.6 / 32.3
+// Below 4096 cells (16^3) nothing was measured.
+static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
+{
+  const bool f16 = s->precision == LBM_F16, aa = s->pattern == LBM_AA;
+  if (s->slab || s->tma || s->n_fluid < 4096 || (!s->compact && s->precision != LBM_F64))
+    return LBM_OK;
+  const double mb = s->state_bytes / 1e6;
+  const bool fronts = mb > (aa && !s->compact ? 95.0 : 85.0);
+  if (aa && ((!s->compact && mb > 60.0 && mb <= 95.0) || (f16 && mb > 33.0)))
+    return LBM_OK;
+  SweepShape h;
+  h.nx = s->g.nx;
+  h.ny = s->g.ny;
+  h.pair = s->precision != LBM_F64;
+  const int words = (s->g.nz + 31) / 32;
+  h.units = (uint32_t)(h.pair ? (words + 1) / 2 : words);
+  h.row_start = s->compact ? row_start.data() : NULL;
+  h.local_first = s->pattern != LBM_PULL;
+  h.plane_bytes = (double)s->state_bytes / s->g.nx;
+  h.resident = 8u * (uint32_t)sm_count(); // all sweep kernels run 7 or 8 blocks per SM
+  if (!sweep_plan(h, fronts, s->sweep))
+    return LBM_OK;
+  const int steps = fronts ? 2 : kSweepMaxSteps;
+  int rc = dev_alloc(s, (void **)&s->sweep_done,
+      sizeof(uint32_t) * sweep_counter(s->sweep, s->g.nx, steps - 1, 0, 0),
+      "the sweep counters");
+  if (rc)
+    return rc;
+  s->sweep.done = s->sweep_done;
+  s->sweep.err = s->dev_err;
+  s->sweep_steps = steps;
+  return LBM_OK;
+}
 
 // slab = 1: flags has nx + 2 planes in x (x fastest); planes 0 and nx + 1
 // are the neighbouring slabs' boundary planes and become ghost planes.
@@ -680,7 +753,7 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
 
   // compact layout: one fluid bit per cell and the storage index of the
   // first fluid cell of every 32-cell word, rows in (x, y) order
-  std::vector<uint32_t> hbits, hbase;
+  std::vector<uint32_t> hbits, hbase, row_start;
   s->compact = compact;
   if (s->compact) {
     const int W = (s->g.nz + 31) / 32;
@@ -696,6 +769,10 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     for (int x = 0; x < s->g.nx; ++x)
       (*s->cplane0)[x] = hbase[(size_t)x * s->g.ny * W];
     (*s->cplane0)[s->g.nx] = run;
+    row_start.resize(rows + 1);
+    for (size_t r = 0; r < rows; ++r)
+      row_start[r] = hbase[r * W];
+    row_start[rows] = run;
     s->g.plane = ((long long)run + pq - 1) / pq * pq;
     if (s->g.plane == 0)
       s->g.plane = pq;
@@ -770,6 +847,8 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     }
   }
 
+  TRY(init_sweep(s, row_start));
+
   {
     // cells of the Zou-He pressure boundary (src/lbm.c:693-700): flag 2 on
     // x = 0 and flag 4 on x = nx - 1, on the interior rows 1..ny-2, 1..nz-2
@@ -797,8 +876,9 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     std::vector<uint2> hwb(hbits.size());
     for (size_t k = 0; k < hwb.size(); ++k)
       hwb[k] = make_uint2(hbits[k], hbase[k]);
-    TRY(dev_alloc(s, (void **)&s->cwb, 2 * nw, "the compact layout's index"));
-    TRYC(cudaMemcpy(s->cwb, hwb.data(), 2 * nw, cudaMemcpyHostToDevice));
+    hwb.push_back(make_uint2(0u, row_start.back())); // a row's end is the next row's start
+    TRY(dev_alloc(s, (void **)&s->cwb, 2 * nw + sizeof(uint2), "the compact layout's index"));
+    TRYC(cudaMemcpy(s->cwb, hwb.data(), 2 * nw + sizeof(uint2), cudaMemcpyHostToDevice));
     s->g.wb = s->cwb;
   }
   Grid gd = s->g; // dense view of the box for the mask build
@@ -971,8 +1051,7 @@ template <class ST> static int pack_all(lbm_solver *s, const double *f)
         (float)(s->precision == LBM_F16 ? s->fp16_scale : 1.0), weight(d));
     CUDA_TRY(cudaGetLastError());
   }
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return LBM_OK;
+  return sync_and_check(s);
 }
 
 template <class ST> static int unpack_all(lbm_solver *s, double *f)
@@ -990,8 +1069,7 @@ template <class ST> static int unpack_all(lbm_solver *s, double *f)
     CUDA_TRY(cudaMemcpyAsync(f + d * plane_host, s->staging, sizeof(double) * plane_host,
         cudaMemcpyDeviceToHost, s->stream));
   }
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return LBM_OK;
+  return sync_and_check(s);
 }
 
 extern "C" int lbm_set_state(lbm_solver *s, const double *f)
@@ -1291,8 +1369,7 @@ static int ref_transfer_aos(lbm_solver *s, void *host, int ref_orient, bool uplo
       CUDA_TRY(cudaMemcpyAsync(hc, dp, nbytes, cudaMemcpyDeviceToHost, s->stream));
     }
   }
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return LBM_OK;
+  return sync_and_check(s);
 }
 
 template <class ST, typename H>
@@ -1333,8 +1410,7 @@ static int ref_transfer(lbm_solver *s, void *host, int ref_orient, bool upload)
       CUDA_TRY(cudaMemcpyAsync(hp + p * gpl, dp, bytes, cudaMemcpyDeviceToHost, s->stream));
     }
   }
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return LBM_OK;
+  return sync_and_check(s);
 }
 
 static int ref_dispatch(lbm_solver *s, void *host, int elem_size, int ref_orient, bool upload)
@@ -1450,6 +1526,7 @@ static int launch_kernel(lbm_solver *s, int x0, int planes, cudaStream_t st, int
     a.c = make_consts<double>(s);
     a.x0 = x0;
     if (s->tma && !brink && whole) {
+      s->err_pending = 1;
       TmaArgs<StoreF64> t;
       t.s = a;
       t.T = s->tma_shape.T;
@@ -1620,28 +1697,64 @@ extern "C" int lbm_set_pressure_bc(lbm_solver *s, double rho_in, double rho_out,
   return LBM_OK;
 }
 
+// Launches a sweep of `steps` steps (even, at most s->sweep_steps).
+static int launch_sweep(lbm_solver *s, int steps)
+{
+  SweepLaunch l;
+  l.g = s->g;
+  l.f = (void *)state_ptr(s);
+  l.mask = s->mask;
+  l.p = s->sweep;
+  l.p.steps = steps;
+  if (!l.p.lag)
+    l.p.blocks = l.p.front * (uint32_t)s->g.nx * (uint32_t)(steps / 2);
+  const bool brink = s->alpha != 0.0 && s->porosity;
+  l.porosity = brink ? s->porosity : NULL;
+  l.force = s->force_on || brink;
+  l.flip = s->pattern == LBM_PULL;
+  CUDA_TRY(cudaMemsetAsync(s->sweep_done, 0,
+      sizeof(uint32_t) * sweep_counter(l.p, s->g.nx, steps - 1, 0, 0), s->stream));
+  s->err_pending = 1;
+  cudaError_t e = s->precision == LBM_F64
+      ? launch_sweep_f64(l, make_consts<double>(s), s->stream)
+      : launch_sweep_x2(s->precision, l, make_consts2(s), s->stream);
+  if (e != cudaSuccess)
+    return fail(LBM_ERR_CUDA, "sweep launch failed: %s", cudaGetErrorString(e));
+  s->launches++;
+  s->steps_done += steps; // even: pull and push end in the lattice they began in
+  return LBM_OK;
+}
+
+// Steps the next launch of lbm_run takes as one sweep when `left` are left;
+// 0: a single step. A sweep begins at a natural (AA, push) or pull state, so
+// an AA state after an odd number of steps takes a single step first.
+static int next_sweep(const lbm_solver *s, int left)
+{
+  if (!s->sweep_steps || left < 2 || s->split || s->bc_on)
+    return 0;
+  if (s->pattern == LBM_AA && (s->steps_done & 1))
+    return 0;
+  if (s->pattern == LBM_PULL && s->alpha != 0.0 && s->porosity)
+    return 0; // no Brinkman term in the pull orientation
+  return std::min(left & ~1, s->sweep_steps);
+}
+
 extern "C" int lbm_run(lbm_solver *s, int steps)
 {
   if (!s || steps < 0)
     return fail(LBM_ERR_ARG, "lbm_run: bad arguments");
   CUDA_TRY(cudaSetDevice(s->device));
   for (int i = 0; i < steps; ++i) {
+    if (const int n = next_sweep(s, steps - i)) {
+      int rc = launch_sweep(s, n);
+      if (rc)
+        return rc;
+      i += n - 1;
+      continue;
+    }
     int rc = launch_one(s, NULL);
     if (rc)
       return rc;
-  }
-  return LBM_OK;
-}
-
-// Reads the kernels' error word after the stream has drained.
-static int check_kernel_error(lbm_solver *s)
-{
-  unsigned int err = 0;
-  CUDA_TRY(cudaMemcpy(&err, s->dev_err, sizeof(err), cudaMemcpyDeviceToHost));
-  if (err) {
-    CUDA_TRY(cudaMemset(s->dev_err, 0, sizeof(err)));
-    return fail(LBM_ERR_CUDA, "a pipelined step kernel gave up waiting for its bulk copies; "
-        "the state is undefined");
   }
   return LBM_OK;
 }
@@ -1650,10 +1763,9 @@ extern "C" int lbm_synchronize(lbm_solver *s)
 {
   if (!s)
     return fail(LBM_ERR_ARG, "lbm_synchronize: NULL solver");
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
   if (s->side)
     CUDA_TRY(cudaStreamSynchronize(s->side));
-  return check_kernel_error(s);
+  return sync_and_check(s);
 }
 
 extern "C" int lbm_run_timed(lbm_solver *s, int steps, double *ms)
@@ -1671,7 +1783,7 @@ extern "C" int lbm_run_timed(lbm_solver *s, int steps, double *ms)
   float t = 0.f;
   CUDA_TRY(cudaEventElapsedTime(&t, s->ev[0], s->ev[1]));
   *ms = t;
-  return check_kernel_error(s);
+  return sync_and_check(s);
 }
 
 extern "C" int lbm_time_launches(lbm_solver *s, int steps, double *ms_sum, int *count,
@@ -1713,7 +1825,7 @@ extern "C" int lbm_time_launches(lbm_solver *s, int steps, double *ms_sum, int *
     return rc;
   if (e != cudaSuccess)
     return fail(LBM_ERR_CUDA, "lbm_time_launches: %s", cudaGetErrorString(e));
-  return check_kernel_error(s);
+  return sync_and_check(s);
 }
 
 template <class ST> static int moments_t(lbm_solver *s, double *q[4])
@@ -1731,8 +1843,7 @@ template <class ST> static int moments_t(lbm_solver *s, double *q[4])
     CUDA_TRY(cudaMemcpyAsync(q[k], s->staging, sizeof(double) * n, cudaMemcpyDeviceToHost,
         s->stream));
   }
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
-  return LBM_OK;
+  return sync_and_check(s);
 }
 
 extern "C" int lbm_moments(lbm_solver *s, double *rho, double *ux, double *uy, double *uz)
@@ -1772,7 +1883,8 @@ extern "C" int lbm_mass_momentum(lbm_solver *s, double out[4], long long *nonfin
   CUDA_TRY(cudaGetLastError());
   double h[kRedVals];
   CUDA_TRY(cudaMemcpyAsync(h, fin, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  if (int rc = sync_and_check(s))
+    return rc;
   for (int k = 0; k < 4; ++k)
     out[k] = h[k];
   long long bad = (long long)h[4];
@@ -1811,7 +1923,8 @@ extern "C" int lbm_compare(lbm_solver *a, lbm_solver *b, double out[6])
       a->ub.oy != b->ub.oy || a->ub.oz != b->ub.oz)
     return fail(LBM_ERR_ARG, "lbm_compare: solvers differ in geometry or device");
   CUDA_TRY(cudaSetDevice(a->device));
-  CUDA_TRY(cudaStreamSynchronize(b->stream));
+  if (int rc = sync_and_check(b))
+    return rc;
   if (a->precision == LBM_F64)
     compare_b<StoreF64>(a, b);
   else if (a->precision == LBM_F32)
@@ -1824,7 +1937,8 @@ extern "C" int lbm_compare(lbm_solver *a, lbm_solver *b, double out[6])
   CUDA_TRY(cudaGetLastError());
   double h[kRedVals];
   CUDA_TRY(cudaMemcpyAsync(h, fin, sizeof(h), cudaMemcpyDeviceToHost, a->stream));
-  CUDA_TRY(cudaStreamSynchronize(a->stream));
+  if (int rc = sync_and_check(a))
+    return rc;
   for (int k = 0; k < 6; ++k)
     out[k] = h[k];
   return LBM_OK;
@@ -1855,7 +1969,8 @@ extern "C" int lbm_objective(lbm_solver *s, double *j)
   CUDA_TRY(cudaGetLastError());
   double h[kRedVals];
   CUDA_TRY(cudaMemcpyAsync(h, fin, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  if (int rc = sync_and_check(s))
+    return rc;
   *j = h[1] > 0 ? h[0] / h[1] : 0.0;
   return LBM_OK;
 }
@@ -2201,7 +2316,8 @@ static int outlet_sums(lbm_solver *s, double *sum, double *count)
   CUDA_TRY(cudaGetLastError());
   double h[kRedVals];
   CUDA_TRY(cudaMemcpyAsync(h, fin, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
-  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  if (int rc = sync_and_check(s))
+    return rc;
   *sum = h[0];
   *count = h[1];
   return LBM_OK;
@@ -2396,7 +2512,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
       ATRY(cudaGetLastError());
       ATRY(cudaMemcpyAsync(grad, s->staging, sizeof(double) * (size_t)s->nx * s->ny * s->nz,
           cudaMemcpyDeviceToHost, s->stream));
-      ATRY(cudaStreamSynchronize(s->stream));
+      RTRY(sync_and_check(s));
     }
     if (info) {
       info[0] = fwd_ms;

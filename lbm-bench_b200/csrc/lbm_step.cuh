@@ -42,6 +42,10 @@ namespace lbm {
 
 constexpr int kStepThreads = 128;
 
+// Bits of a solver's kernel error word.
+constexpr unsigned kErrBulkCopy = 1u;  // a pipelined step's bulk copy did not arrive
+constexpr unsigned kErrSweepWait = 2u; // a sweep's wait for an earlier step ran out
+
 template <class ST> struct StepArgs {
   using S = typename ST::S;
   using V = typename ST::V;

@@ -235,4 +235,50 @@ cudaError_t launch_step_cp_f64(int kind, bool force, const StepArgs<StoreF64> &a
   return launch_cp<StoreF64>(kind, force, a, grid, block, st);
 }
 
+template <class BODY> static cudaError_t go_sweep(const typename BODY::Args &a, cudaStream_t st)
+{
+  sweep_kernel<BODY><<<a.p.blocks, kStepThreads, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <bool FORCE, bool FLIP>
+static cudaError_t pick_sweep(const SweepLaunch &l, const Consts<double> &c, cudaStream_t st)
+{
+  using ST = StoreF64;
+  SweepArgsD<ST> a;
+  a.g = l.g;
+  a.src = (const double *)l.f;
+  a.dst = (double *)l.f;
+  a.mask = l.mask;
+  a.c = c;
+  a.p = l.p;
+  a.porosity = l.porosity;
+  const bool fronts = l.p.lag > 0;
+  if (!l.g.wb) {
+    if constexpr (FORCE && !FLIP)
+      if (l.porosity)
+        return fronts ? go_sweep<SweepDense<ST, true, false, true, true>>(a, st)
+                      : go_sweep<SweepDense<ST, true, false, true, false>>(a, st);
+    return fronts ? go_sweep<SweepDense<ST, FORCE, FLIP, false, true>>(a, st)
+                  : go_sweep<SweepDense<ST, FORCE, FLIP, false, false>>(a, st);
+  }
+  const bool zper = (l.g.per & 4) != 0;
+  const bool off32 = (unsigned long long)Q * (unsigned long long)l.g.plane < (1ull << 32);
+  if (!fronts) // the lattice fits the L2, so its offsets fit 32 bits
+    return zper ? go_sweep<SweepCp<ST, FORCE, FLIP, true, false, uint32_t>>(a, st)
+                : go_sweep<SweepCp<ST, FORCE, FLIP, false, false, uint32_t>>(a, st);
+  if (off32)
+    return zper ? go_sweep<SweepCp<ST, FORCE, FLIP, true, true, uint32_t>>(a, st)
+                : go_sweep<SweepCp<ST, FORCE, FLIP, false, true, uint32_t>>(a, st);
+  return zper ? go_sweep<SweepCp<ST, FORCE, FLIP, true, true, uint64_t>>(a, st)
+              : go_sweep<SweepCp<ST, FORCE, FLIP, false, true, uint64_t>>(a, st);
+}
+
+cudaError_t launch_sweep_f64(const SweepLaunch &l, const Consts<double> &c, cudaStream_t st)
+{
+  if (l.flip)
+    return l.force ? pick_sweep<true, true>(l, c, st) : pick_sweep<false, true>(l, c, st);
+  return l.force ? pick_sweep<true, false>(l, c, st) : pick_sweep<false, false>(l, c, st);
+}
+
 } // namespace lbm

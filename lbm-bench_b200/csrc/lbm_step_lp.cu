@@ -8,6 +8,7 @@
 #include "lbm_step_x2s.cuh"
 #include "lbm_step_x4s.cuh"
 #include "lbm_step_cp2.cuh"
+#include "lbm_sweep_x2.cuh"
 
 namespace lbm {
 
@@ -161,6 +162,48 @@ cudaError_t launch_step_cp2_f16(int kind, bool force, const StepArgs2<StoreF16> 
     cudaStream_t st)
 {
   return launch_cp2<StoreF16>(kind, force, a, st);
+}
+
+template <class BODY> static cudaError_t go_sweep(const typename BODY::Args &a, cudaStream_t st)
+{
+  sweep_kernel<BODY><<<a.p.blocks, kStepThreads, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <class ST, bool FORCE, bool FLIP>
+static cudaError_t pick_sweep(const SweepLaunch &l, const Consts2 &c, cudaStream_t st)
+{
+  SweepArgs2<ST> a;
+  a.g = l.g;
+  a.src = (const typename ST::S *)l.f;
+  a.dst = (typename ST::S *)l.f;
+  a.mask = l.mask;
+  a.c = c;
+  a.p = l.p;
+  const bool zper = (l.g.per & 4) != 0;
+  const bool off32 = (unsigned long long)Q * (unsigned long long)l.g.plane < (1ull << 32);
+  if (l.p.lag == 0) // the lattice fits the L2, so its offsets fit 32 bits
+    return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, false, uint32_t>>(a, st)
+                : go_sweep<SweepCp2<ST, FORCE, FLIP, false, false, uint32_t>>(a, st);
+  if (off32)
+    return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, true, uint32_t>>(a, st)
+                : go_sweep<SweepCp2<ST, FORCE, FLIP, false, true, uint32_t>>(a, st);
+  return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, true, uint64_t>>(a, st)
+              : go_sweep<SweepCp2<ST, FORCE, FLIP, false, true, uint64_t>>(a, st);
+}
+
+template <class ST>
+static cudaError_t launch_sweep(const SweepLaunch &l, const Consts2 &c, cudaStream_t st)
+{
+  if (l.flip)
+    return l.force ? pick_sweep<ST, true, true>(l, c, st) : pick_sweep<ST, false, true>(l, c, st);
+  return l.force ? pick_sweep<ST, true, false>(l, c, st) : pick_sweep<ST, false, false>(l, c, st);
+}
+
+cudaError_t launch_sweep_x2(int precision, const SweepLaunch &l, const Consts2 &c,
+    cudaStream_t st)
+{
+  return precision == kF32 ? launch_sweep<StoreF32>(l, c, st) : launch_sweep<StoreF16>(l, c, st);
 }
 
 } // namespace lbm
