@@ -602,9 +602,9 @@ static int sync_and_check(lbm_solver *s)
 // ---------------------------------------------------------------------------
 
 // Whether, and in which order, a solver runs sweeps, and their plan. The
-// lines (lattice bytes, or cells) are where sweeps stop to win over single
-// steps; us per step, single steps / step-major / fronts, channels of 64 x 64
-// planes on a B200:
+// lines (lattice bytes) lie where one order or single steps begin to win; us
+// per step, single steps / step-major / fronts, channels of 64 x 64 planes on a
+// B200:
 //   compact FP64 AA    43 MB 12.4 / 9.6 / 14.9   65 MB 16.6 / 14.3 / 19.6
 //                      87 MB 25.8 / 24.6 / 24.3   108 MB 39.0 / 37.2 / 29.7
 //   compact FP64 pull  43 MB 14.4 / 9.6 / 14.2   87 MB 33.5 / 24.9 / 24.5
@@ -613,17 +613,28 @@ static int sync_and_check(lbm_solver *s)
 //   compact FP16 AA    22 MB 13.4 / 11.7 / 16.9   33 MB 17.5 / 17.4 / 22.6
 //                      43 MB 22.2 / 23.1 / 28.4   97 MB 50.0 / 55.4 / 57.9
 //   compact FP16 pull  43 MB 26.7 / 22.9 / 27.4   97 MB 57.5 / 54.5 / 57.3
-//   dense FP64 AA      43 MB 12.4 / 11.2 / 16.0   65 MB 16.5 / 16.9 / 21.3
-//                      87 MB 23.6 / 25.9 / 27.5   108 MB 35.8 / 37.6 / 32.3
+//   dense FP64 AA      65 MB 16.7 / 13.9 / 18.5   87 MB 23.6 / 21.8 / 23.0
+//                      108 MB 35.8 / 33.1 / 27.7
+//   dense FP64 push    65 MB 29.2 / 13.8 / 19.0   87 MB 40.3 / 22.2 / 23.5
+//   dense FP32 AA      65 MB 20.6 / 16.7 / 21.1   87 MB 33.9 / 25.6 / 25.7
+//   dense FP16 AA      65 MB 44.1 / 33.1 / 36.9   97 MB 69.0 / 54.5 / 53.9
+//   dense FP16 pull    65 MB 36.9 / 34.4 / 36.4   97 MB 53.0 / 55.8 / 52.3
+// and at 256^3 (20% solid) in ms, single / fronts: compact FP16 AA 0.274 /
+// 0.305, pull 0.316 / 0.304, push 0.356 / 0.305; dense FP16 pull 0.302 / 0.321
+// (its single steps read rows of whole 64-cell segments in aligned pairs).
 // Below 4096 cells (16^3) nothing was measured.
 static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
 {
-  const bool f16 = s->precision == LBM_F16, aa = s->pattern == LBM_AA;
-  if (s->slab || s->tma || s->n_fluid < 4096 || (!s->compact && s->precision != LBM_F64))
+  if (s->slab || s->tma || s->n_fluid < 4096)
+    return LBM_OK;
+  // the dense layout's sweeps address the 19 planes with 32-bit offsets
+  if (!s->compact && (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return LBM_OK;
   const double mb = s->state_bytes / 1e6;
-  const bool fronts = mb > (aa && !s->compact ? 95.0 : 85.0);
-  if (aa && ((!s->compact && mb > 60.0 && mb <= 95.0) || (f16 && mb > 33.0)))
+  const bool fronts = mb > 85.0;
+  if (s->precision == LBM_F16 &&
+      (s->compact ? s->pattern == LBM_AA && mb > 33.0
+                  : s->pattern == LBM_PULL && fronts && s->g.nz % 64 == 0))
     return LBM_OK;
   SweepShape h;
   h.nx = s->g.nx;

@@ -173,13 +173,23 @@ template <class BODY> static cudaError_t go_sweep(const typename BODY::Args &a, 
 template <class ST, bool FORCE, bool FLIP>
 static cudaError_t pick_sweep(const SweepLaunch &l, const Consts2 &c, cudaStream_t st)
 {
-  SweepArgs2<ST> a;
+  SweepArgsD2<ST> a;
   a.g = l.g;
   a.src = (const typename ST::S *)l.f;
   a.dst = (typename ST::S *)l.f;
   a.mask = l.mask;
   a.c = c;
   a.p = l.p;
+  a.porosity = l.porosity;
+  if (!l.g.wb) {
+    const bool fronts = l.p.lag > 0;
+    if constexpr (FORCE && !FLIP)
+      if (l.porosity)
+        return fronts ? go_sweep<SweepDense2<ST, true, false, true, true>>(a, st)
+                      : go_sweep<SweepDense2<ST, true, false, true, false>>(a, st);
+    return fronts ? go_sweep<SweepDense2<ST, FORCE, FLIP, false, true>>(a, st)
+                  : go_sweep<SweepDense2<ST, FORCE, FLIP, false, false>>(a, st);
+  }
   const bool zper = (l.g.per & 4) != 0;
   const bool off32 = (unsigned long long)Q * (unsigned long long)l.g.plane < (1ull << 32);
   if (l.p.lag == 0) // the lattice fits the L2, so its offsets fit 32 bits

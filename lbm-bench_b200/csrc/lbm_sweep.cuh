@@ -83,6 +83,15 @@ template <bool STREAM, typename S> __device__ __forceinline__ void sweep_store(S
     *p = v;
 }
 
+// The same value, unknown to the compiler: the scatter of an in-place step
+// computes its offsets again (a multiply-add each) instead of keeping the
+// gather's, which are the same set, live across the collision (spills).
+__device__ __forceinline__ uint32_t recompute(uint32_t v)
+{
+  asm volatile("" : "+r"(v));
+  return v;
+}
+
 // BODY: local(a, item, tid, wait) and shifted(a, item, tid, wait) update one
 // block's share of an item. They look up indices and masks, which no step
 // changes, then call wait() (block-wide: one warp polls) and only then touch
@@ -208,7 +217,7 @@ struct SweepCp {
   {
     const SweepCells sc = sweep_cells(a.g, it);
     const uint32_t i = it.b * kStepThreads + (uint32_t)tid;
-    const uint32_t cell = i < sc.n0 ? sc.c0 + i : sc.c1 + (i - sc.n0);
+    uint32_t cell = i < sc.n0 ? sc.c0 + i : sc.c1 + (i - sc.n0);
     if (FRONTS && kLocalFirst)
       sweep_prefetch<kStepThreads>(a.g, a.src, a.mask, it, tid);
     wait();
@@ -221,6 +230,7 @@ struct SweepCp {
       v[d] = ST::decode(a.src[el(a, d, cell)], a.c.inv_scale);
     V o[Q];
     collide<V, false>(v, o, a.c, V(0));
+    cell = recompute(cell);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const bool bb = (mask >> d) & 1u;
@@ -270,6 +280,7 @@ struct SweepCp {
     }
     V o[Q];
     collide<V, false>(v, o, a.c, V(0));
+    cell = recompute(cell);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const bool bb = (mask >> d) & 1u;
@@ -280,14 +291,18 @@ struct SweepCp {
   }
 };
 
-// 72 registers: 7 blocks per SM (AA / pull at 256^3: 8 0.727 / 0.660 ms with
-// spills, 7 0.608 / 0.645, 6 0.607 / 0.662).
+// Blocks per SM, from AA and push / pull at 256^3: 8 0.564 / 0.585 ms, 7 0.529 /
+// 0.601, 6 0.542 / 0.638.
 #ifndef LBM_MINB_SWEEP_DENSE
 #define LBM_MINB_SWEEP_DENSE 7
 #endif
+#ifndef LBM_MINB_SWEEP_DENSE_PULL
+#define LBM_MINB_SWEEP_DENSE_PULL 8
+#endif
 
 // FP64, dense layout, one cell per thread (step_kernel). BRINK adds the
-// Brinkman term of a.porosity.
+// Brinkman term of a.porosity. Offsets of the 19 planes fit 32 bits (checked
+// at planning).
 template <class ST> struct SweepArgsD : SweepArgs<ST> {
   const float *porosity;
 };
@@ -295,12 +310,12 @@ template <class ST> struct SweepArgsD : SweepArgs<ST> {
 template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct SweepDense {
   using Args = SweepArgsD<ST>;
   using V = typename ST::V;
-  static constexpr int kMinBlocks = LBM_MINB_SWEEP_DENSE;
+  static constexpr int kMinBlocks = FLIP ? LBM_MINB_SWEEP_DENSE_PULL : LBM_MINB_SWEEP_DENSE;
   static constexpr bool kLocalFirst = !FLIP;
 
-  __device__ static long long pl(const Args &a, int plane)
+  __device__ static uint32_t el(const Args &a, int plane, uint32_t i)
   {
-    return (FLIP ? inv(plane) : plane) * a.g.plane;
+    return (uint32_t)(FLIP ? inv(plane) : plane) * (uint32_t)a.g.plane + i;
   }
 
   template <bool SHIFTED, class WAIT>
@@ -338,19 +353,18 @@ template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct Sweep
     if (!SHIFTED) {
 #pragma unroll
       for (int d = 0; d < Q; ++d)
-        v[d] = ST::decode(a.src[pl(a, d) + cell], a.c.inv_scale);
+        v[d] = ST::decode(a.src[el(a, d, cell)], a.c.inv_scale);
     } else if (!__any_sync(__activemask(), (mask & 0x7FFFFu) != 0u)) {
 #pragma unroll
       for (int d = 0; d < Q; ++d)
-        v[d] = ST::decode(a.src[pl(a, inv(d)) + (uint32_t)(cell + of.at(inv(d)))],
+        v[d] = ST::decode(a.src[el(a, inv(d), cell + of.at(inv(d)))],
             a.c.inv_scale);
     } else {
 #pragma unroll
       for (int d = 0; d < Q; ++d) {
         const bool back = (mask >> inv(d)) & 1u;
-        const typename ST::S *p = back ? a.src + pl(a, d) + cell
-                                       : a.src + pl(a, inv(d)) + (uint32_t)(cell + of.at(inv(d)));
-        v[d] = ST::decode(*p, a.c.inv_scale);
+        const uint32_t o = back ? el(a, d, cell) : el(a, inv(d), cell + of.at(inv(d)));
+        v[d] = ST::decode(a.src[o], a.c.inv_scale);
       }
     }
     V kappa = V(0);
@@ -358,13 +372,13 @@ template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct Sweep
       kappa = a.c.alpha * (V(1.0) - V(a.porosity[cell]));
     V o[Q];
     collide<V, BRINK>(v, o, a.c, kappa);
+    cell = recompute(cell);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const bool bb = (mask >> d) & 1u;
       const V w = FORCE ? o[d] + (bb ? a.c.force[inv(d)] : a.c.force[d]) : o[d];
-      typename ST::S *p = !SHIFTED || bb ? a.dst + pl(a, inv(d)) + cell
-                                         : a.dst + pl(a, d) + (uint32_t)(cell + of.at(d));
-      sweep_store<FRONTS && kLast>(p, ST::encode(w, a.c.scale));
+      const uint32_t o = !SHIFTED || bb ? el(a, inv(d), cell) : el(a, d, cell + of.at(d));
+      sweep_store<FRONTS && kLast>(a.dst + o, ST::encode(w, a.c.scale));
     }
   }
   template <class WAIT>

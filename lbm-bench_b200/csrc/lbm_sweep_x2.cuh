@@ -1,13 +1,16 @@
-// Sweeps (lbm_sweep.cuh) of the reduced-precision storage modes in the
-// compact layout: two cells per thread with the pair arithmetic, operation for
-// operation that of the single-step kernels (lbm_step_cp2.cuh).
+// Sweeps (lbm_sweep.cuh) of the reduced-precision storage modes, two cells per
+// thread with the pair arithmetic, operation for operation that of the
+// single-step kernels (lbm_step_x2.cuh, lbm_step_cp2.cuh).
 //
-// FP32 at 256^3 (20% solid): 0.310 ms a step (AA, push) and 0.314 (pull)
-// against 0.357, 0.439 and 0.388 in single steps. HBM is then at 48% of its
-// peak; what bounds it is the L1's request rate to the L2 (66% busy: a warp's
-// store is 128 bytes, half of an FP64 one) and instruction issue (61%).
-// FP16 halves the bytes but not the requests and takes the same 0.310 ms, so
-// its AA steps (0.274 ms) sweep only where the launch gaps count.
+// At 256^3 (20% solid), ms a step, sweeps / single steps:
+//   compact FP32  AA 0.303 / 0.357   pull 0.305 / 0.388   push 0.303 / 0.439
+//   dense FP32    AA 0.310 / 0.487   pull 0.330 / 0.406   push 0.310 / 0.619
+//   dense FP16    AA 0.310 / 0.353   push 0.309 / 0.417
+// HBM is then at 48% of its peak; what bounds a sweep is the L1's request rate
+// to the L2 (66% busy: a warp's store is 128 bytes, half of an FP64 one) and
+// instruction issue (61%). FP16 halves the bytes but not the requests and
+// takes the same time, so compact FP16 AA (0.274 in single steps) sweeps only
+// where the launch gaps count.
 #pragma once
 
 #include "lbm_step_cp2.cuh"
@@ -24,7 +27,7 @@ template <class ST> struct SweepArgs2 {
   SweepPlan p;
 };
 
-// 64 registers: 8 blocks per SM (9: 0.330 ms, 7: 0.313, 6: 0.327; 8: 0.310).
+// 64 registers: 8 blocks per SM (FP32 AA 9: 0.330 ms, 8: 0.310, 7: 0.313, 6: 0.327).
 #ifndef LBM_MINB_SWEEP_CP2
 #define LBM_MINB_SWEEP_CP2 8
 #endif
@@ -55,6 +58,7 @@ struct SweepCp2 {
       f[d] = PT::dec(*reinterpret_cast<const P *>(a.src + el(a, d, cell)));
     float2 o[Q];
     collide2<false>(f, o, a.c, f2(0.f), nullptr);
+    cell = recompute(cell);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const float2 v = FORCE ? add_force2(o[d], d, m.x, m.y, a.c.force) : o[d];
@@ -160,6 +164,8 @@ struct SweepCp2 {
     }
     float2 o[Q];
     collide2<false>(f, o, a.c, make_float2(0.0f, 0.0f), nullptr);
+    cell0 = recompute(cell0);
+    cell1 = recompute(cell1);
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const float2 v = FORCE ? add_force2(o[d], d, m0, m1, a.c.force) : o[d];
@@ -169,6 +175,155 @@ struct SweepCp2 {
         sweep_store<FRONTS && kLocalFirst>(q0, PT::enc1(v.x));
       if (fl1)
         sweep_store<FRONTS && kLocalFirst>(q1, PT::enc1(v.y));
+    }
+  }
+};
+
+// Blocks per SM, from AA / pull at 256^3: FP32 8 0.316 / 0.355 ms, 7 0.310 /
+// 0.330, 6 0.324 / 0.360; FP16 0.310 / 0.321, 0.313 / 0.325, 0.325 / 0.330.
+#ifndef LBM_MINB_SWEEP_X2
+#define LBM_MINB_SWEEP_X2 7
+#endif
+#ifndef LBM_MINB_SWEEP_X2_F16
+#define LBM_MINB_SWEEP_X2_F16 8
+#endif
+
+// Dense layout. Local step: cells z and z + 1 of one row per thread, one
+// aligned pair access per plane. Shifted step: cells z and z + 32, so that
+// every access of a warp is 32 consecutive elements and, away from walls and
+// row ends, the second cell's is the first's address plus a constant (as
+// z-adjacent pairs it needs twice the addresses, and 250-500 bytes of spills).
+// BRINK adds the Brinkman term of a.porosity. Offsets of the 19 planes fit 32
+// bits (checked at planning).
+template <class ST> struct SweepArgsD2 : SweepArgs2<ST> {
+  const float *porosity;
+};
+
+template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct SweepDense2 {
+  using Args = SweepArgsD2<ST>;
+  using PT = PairOf<ST>;
+  using S = typename PT::S;
+  using P = typename PT::P;
+  static constexpr int kMinBlocks = sizeof(S) == 2 ? LBM_MINB_SWEEP_X2_F16 : LBM_MINB_SWEEP_X2;
+  static constexpr bool kLocalFirst = !FLIP;
+
+  __device__ static uint32_t el(const Args &a, int plane, uint32_t i)
+  {
+    return (uint32_t)(FLIP ? inv(plane) : plane) * (uint32_t)a.g.plane + i;
+  }
+
+  template <class WAIT>
+  __device__ __forceinline__ static void local(const Args &a, const SweepItem &it, int tid,
+      WAIT &&wait)
+  {
+    const Grid &g = a.g;
+    int y;
+    uint32_t unit;
+    uint32_t cell = 0;
+    uint2 m = make_uint2(kSolidBit, kSolidBit);
+    const bool row_ok = sweep_unit(a.p, g.ny, it, tid >> 5, y, unit);
+    const int z = (int)(64u * unit) + 2 * (tid & 31);
+    if (row_ok && z < g.nz) {
+      // the pair starts at an even element; a cell z + 1 = nz is padding and
+      // carries the wall bit
+      cell = cell_index(g, it.x, y, z);
+      m = *reinterpret_cast<const uint2 *>(a.mask + cell);
+    }
+    if (FRONTS && kLocalFirst && tid <= Q && it.x + 1 < g.nx) {
+      const uint32_t lo = cell_index(g, it.x + 1, it.r0, 0) + it.b * 2 * kStepThreads;
+      const uint32_t hi = min(lo + 2 * kStepThreads, cell_index(g, it.x + 1, it.r1, 0));
+      if (lo < hi) {
+        if (tid < Q)
+          l2_prefetch_bytes(a.src + tid * g.plane, (unsigned long long)lo * sizeof(S),
+              (unsigned long long)hi * sizeof(S));
+        else
+          l2_prefetch_bytes(a.mask, lo * 4ull, hi * 4ull);
+      }
+    }
+    wait();
+    if (m.x & m.y & kSolidBit)
+      return;
+    float2 f[Q];
+#pragma unroll
+    for (int d = 0; d < Q; ++d)
+      f[d] = PT::dec(*reinterpret_cast<const P *>(a.src + el(a, d, cell)));
+    float2 kappa = f2(0.f);
+    if (BRINK) {
+      const float2 por = *reinterpret_cast<const float2 *>(a.porosity + cell);
+      kappa = make_float2(a.c.alpha * (1.f - por.x), a.c.alpha * (1.f - por.y));
+    }
+    float2 o[Q];
+    collide2<BRINK>(f, o, a.c, kappa, nullptr);
+    cell = recompute(cell);
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+      // a wall cell's own slot is never read: both cells are written
+      const float2 v = FORCE ? add_force2(o[d], d, m.x, m.y, a.c.force) : o[d];
+      sweep_store<FRONTS && !kLocalFirst>(reinterpret_cast<P *>(a.dst + el(a, inv(d), cell)),
+          PT::enc(v));
+    }
+  }
+
+  template <class WAIT>
+  __device__ __forceinline__ static void shifted(const Args &a, const SweepItem &it, int tid,
+      WAIT &&wait)
+  {
+    constexpr bool kStream = FRONTS && kLocalFirst;
+    const Grid &g = a.g;
+    int y;
+    uint32_t unit;
+    uint32_t cell = 0, m0 = kSolidBit, m1 = kSolidBit;
+    const bool row_ok = sweep_unit(a.p, g.ny, it, tid >> 5, y, unit);
+    const int z = (int)(64u * unit) + (tid & 31);
+    if (row_ok && z < g.nz) {
+      cell = cell_index(g, it.x, y, z);
+      m0 = __ldg(a.mask + cell);
+      if (z + 32 < g.nz)
+        m1 = __ldg(a.mask + cell + 32u);
+    }
+    wait();
+    const bool fl0 = !(m0 & kSolidBit), fl1 = !(m1 & kSolidBit);
+    if (!fl0 && !fl1)
+      return;
+    const Offs of = make_offs(g, it.x, y, z);
+    // z neighbours of the second cell: it can only wrap at the row's end,
+    // the first one only at its start (a row that ends in the first 32 cells
+    // has no second cell)
+    Offs of1 = of;
+    of1.zm = 0u - 1u;
+    of1.zp = ((g.per >> 2) & 1) && z + 32 == g.nz - 1 ? 0u - (uint32_t)(g.nz - 1) : 1u;
+    auto ld = [&](bool fl, uint32_t o) { return fl ? PT::dec1(a.src[o]) : 0.0f; };
+    const bool links = __any_sync(__activemask(), ((m0 | m1) & 0x7FFFFu) != 0u);
+    float2 f[Q];
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+      const int e = inv(d); // x - c_d = x + c_e
+      uint32_t p0 = el(a, inv(d), cell + of.at(e));
+      uint32_t p1 = cz(e) == 0 ? p0 + 32u : el(a, inv(d), cell + 32u + of1.at(e));
+      if (links) {
+        p0 = ((m0 >> e) & 1u) ? el(a, d, cell) : p0;
+        p1 = ((m1 >> e) & 1u) ? el(a, d, cell + 32u) : p1;
+      }
+      f[d] = make_float2(ld(fl0, p0), ld(fl1, p1));
+    }
+    float2 kappa = f2(0.f);
+    if (BRINK)
+      kappa = make_float2(fl0 ? a.c.alpha * (1.f - a.porosity[cell]) : 0.f,
+          fl1 ? a.c.alpha * (1.f - a.porosity[cell + 32u]) : 0.f);
+    float2 o[Q];
+    collide2<BRINK>(f, o, a.c, kappa, nullptr);
+    cell = recompute(cell);
+#pragma unroll
+    for (int d = 0; d < Q; ++d) {
+      const float2 v = FORCE ? add_force2(o[d], d, m0, m1, a.c.force) : o[d];
+      uint32_t q0 = el(a, d, cell + of.at(d));
+      uint32_t q1 = cz(d) == 0 ? q0 + 32u : el(a, d, cell + 32u + of1.at(d));
+      q0 = ((m0 >> d) & 1u) ? el(a, inv(d), cell) : q0;
+      q1 = ((m1 >> d) & 1u) ? el(a, inv(d), cell + 32u) : q1;
+      if (fl0)
+        sweep_store<kStream>(a.dst + q0, PT::enc1(v.x));
+      if (fl1)
+        sweep_store<kStream>(a.dst + q1, PT::enc1(v.y));
     }
   }
 };
