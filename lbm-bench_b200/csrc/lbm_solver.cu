@@ -60,8 +60,11 @@ struct lbm_solver {
   uint32_t *mask;
   float *porosity;
   double alpha;
-  double *staging; // one dense plane, nx*ny*nz doubles
-  void *pstaging;  // one plane of the reference's padded layout (allocated on first use)
+  double *staging; // transfer staging: at least one dense plane (nx*ny*nz doubles)
+  size_t staging_bytes;
+  cudaStream_t bus; // host copies of pipelined transfers, created on first use
+  cudaEvent_t bus_ev[2], conv_ev[2];
+  void *pstaging;  // x planes of the reference's padded AoS layout (allocated on first use)
   size_t pstaging_bytes;
   double *red;     // reduction partials
   long long n_fluid;
@@ -288,56 +291,53 @@ __device__ __forceinline__ long long dense_index(const UserBox &u, int x, int y,
   return ((long long)x * u.ny + y) * u.nz + z;
 }
 
-// Dense plane d (caller layout) -> device state in orientation `orient`.
-template <class ST>
-__global__ void pack_plane_kernel(Grid g, UserBox u, int d, int orient,
-    const double *__restrict__ dense, typename ST::S *state, const uint32_t *__restrict__ mask,
-    float scale, double wd)
+// Transfers work on slices: one x plane of one direction, ny x nz values, in
+// the order of the caller's array (slice i: direction i / nx, plane i % nx), so
+// any range of slices is one contiguous piece of it. One launch takes a chunk
+// of slices; see stream_slices.
+__device__ __forceinline__ double weight_of(int d)
 {
-  using V = typename ST::V;
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int x = blockIdx.z;
-  if (z >= u.nz || y >= u.ny)
-    return;
-  uint32_t cell, m;
-  if (!locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m))
-    return;
-  const Nbr nb = make_nbr(g, x + u.ox, y + u.oy, z + u.oz, cell);
-  int p;
-  uint32_t c;
-  state_slot(orient, d, m, cell, nb, p, c);
-  double v = dense[dense_index(u, x, y, z)];
-  if (ST::kShifted)
-    v -= wd;
-  ST::store(state + (long long)p * g.plane + c, (V)v, (V)scale);
+  const int c = wclass(d);
+  return c == 0 ? 1.0 / 3.0 : c == 1 ? 1.0 / 18.0 : 1.0 / 36.0;
 }
 
-// Device state -> dense plane d (caller layout); obstacles get 0.
-template <class ST>
-__global__ void unpack_plane_kernel(Grid g, UserBox u, int d, int orient,
-    double *__restrict__ dense, const typename ST::S *state, const uint32_t *__restrict__ mask,
-    float inv_scale, double wd)
+// Slices i0 .. i0 + gridDim.z - 1 (UP: caller -> state in orientation
+// `orient`; else state -> caller, obstacles as 0).
+template <class ST, bool UP>
+__global__ void dense_slices_kernel(Grid g, UserBox u, int i0, int orient,
+    double *__restrict__ chunk, typename ST::S *state, const uint32_t *__restrict__ mask,
+    float scale)
 {
   using V = typename ST::V;
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int x = blockIdx.z;
+  const int i = i0 + (int)blockIdx.z;
+  const int d = i / u.nx, x = i - d * u.nx;
   if (z >= u.nz || y >= u.ny)
     return;
+  double *value = chunk + ((long long)blockIdx.z * u.ny + y) * u.nz + z;
   uint32_t cell, m;
   if (!locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m)) {
-    dense[dense_index(u, x, y, z)] = 0.0;
+    if (!UP)
+      *value = 0.0;
     return;
   }
   const Nbr nb = make_nbr(g, x + u.ox, y + u.oy, z + u.oz, cell);
   int p;
   uint32_t c;
   state_slot(orient, d, m, cell, nb, p, c);
-  double v = (double)ST::load(state + (long long)p * g.plane + c, d, (V)inv_scale);
-  if (ST::kShifted)
-    v += wd;
-  dense[dense_index(u, x, y, z)] = v;
+  typename ST::S *slot = state + (long long)p * g.plane + c;
+  if (UP) {
+    double v = *value;
+    if (ST::kShifted)
+      v -= weight_of(d);
+    ST::store(slot, (V)v, (V)scale);
+  } else {
+    double v = (double)ST::load(slot, d, (V)scale);
+    if (ST::kShifted)
+      v += weight_of(d);
+    *value = v;
+  }
 }
 
 // Density and momentum of one fluid cell in FP64. For shifted storage the
@@ -365,26 +365,31 @@ __device__ __forceinline__ void cell_moments(const Grid &g, const typename ST::S
   }
 }
 
-// quantity: 0 rho, 1 ux, 2 uy, 3 uz (momentum) -> dense cell array
+// Density and momentum of x planes x0 .. x0 + gridDim.z - 1 into four arrays
+// of gridDim.z planes, `stride` values apart: the populations are read once
+// for all four.
 template <class ST>
-__global__ void moments_kernel(Grid g, UserBox u, int orient, int quantity,
-    const typename ST::S *state, const uint32_t *__restrict__ mask, float inv_scale, double *out)
+__global__ void moments_kernel(Grid g, UserBox u, int x0, int orient,
+    const typename ST::S *state, const uint32_t *__restrict__ mask, float inv_scale, double *out,
+    long long stride)
 {
   const int z = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int x = blockIdx.z;
+  const int x = x0 + (int)blockIdx.z;
   if (z >= u.nz || y >= u.ny)
     return;
   uint32_t cell, m;
-  double r = 0.0;
+  double rho = 0.0, jx = 0.0, jy = 0.0, jz = 0.0;
   if (locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m)) {
     const Nbr nb = make_nbr(g, x + u.ox, y + u.oy, z + u.oz, cell);
-    double rho, jx, jy, jz;
     bool fin;
     cell_moments<ST>(g, state, orient, m, cell, nb, inv_scale, rho, jx, jy, jz, fin);
-    r = quantity == 0 ? rho : quantity == 1 ? jx : quantity == 2 ? jy : jz;
   }
-  out[dense_index(u, x, y, z)] = r;
+  double *o = out + ((long long)blockIdx.z * u.ny + y) * u.nz + z;
+  o[0] = rho;
+  o[stride] = jx;
+  o[2 * stride] = jy;
+  o[3 * stride] = jz;
 }
 
 constexpr int kRedThreads = 256;
@@ -556,6 +561,14 @@ static void free_all(lbm_solver *s)
     cudaEventDestroy(s->join_ev);
   if (s->side)
     cudaStreamDestroy(s->side);
+  for (int b = 0; b < 2; ++b) {
+    if (s->bus_ev[b])
+      cudaEventDestroy(s->bus_ev[b]);
+    if (s->conv_ev[b])
+      cudaEventDestroy(s->conv_ev[b]);
+  }
+  if (s->bus)
+    cudaStreamDestroy(s->bus);
   if (s->ev[0])
     cudaEventDestroy(s->ev[0]);
   if (s->ev[1])
@@ -822,8 +835,13 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
   if (pattern != LBM_AA)
     TRY(dev_alloc(s, &s->buf[1], s->state_bytes, "the second population lattice"));
   TRY(dev_alloc(s, (void **)&s->mask, (size_t)s->g.plane * 4, "the link masks"));
-  TRY(dev_alloc(s, (void **)&s->staging, sizeof(double) * (size_t)nx * ny * nz,
-      "the transfer plane"));
+  {
+    // one dense plane, or a whole small (padded) state up to 64 MB
+    const size_t all = sizeof(double) * Q * (size_t)(nx + 2) * (ny + 2) * (nz + 2);
+    s->staging_bytes = std::max(sizeof(double) * (size_t)nx * ny * nz,
+        std::min(all, (size_t)64 << 20));
+    TRY(dev_alloc(s, (void **)&s->staging, s->staging_bytes, "the transfer staging"));
+  }
   TRY(dev_alloc(s, (void **)&s->red, sizeof(double) * kRedVals * (kRedBlocks + 1),
       "reduction partials"));
   TRYC(cudaMemsetAsync(s->buf[0], 0, s->state_bytes, s->stream));
@@ -1046,41 +1064,153 @@ static void user_launch_shape(const lbm_solver *s, dim3 &grid, dim3 &block)
   cell_launch_shape(gu, grid, block);
 }
 
-template <class ST> static int pack_all(lbm_solver *s, const double *f)
+// At least `bytes` of device staging.
+static int need_staging(lbm_solver *s, size_t bytes)
+{
+  if (s->staging_bytes >= bytes)
+    return LBM_OK;
+  CUDA_TRY(cudaStreamSynchronize(s->stream));
+  cudaFree(s->staging);
+  s->staging = NULL;
+  s->dev_bytes -= s->staging_bytes;
+  s->staging_bytes = 0;
+  int rc = dev_alloc(s, (void **)&s->staging, bytes, "the transfer staging");
+  if (!rc)
+    s->staging_bytes = bytes;
+  return rc;
+}
+
+// Moves `count` slices of `slice` bytes between the solver and the host in
+// chunks: kernel(i0, n, dev) converts n slices on the solver's stream,
+// copy(i0, n, dev, stream) moves them over the bus. Chunks alternate between
+// the halves of the staging buffer with the copies on a stream of their own,
+// so the conversion of one chunk runs under the copy of another; a small
+// transfer is one kernel and one copy. (One plane at a time through one buffer,
+// the bus idled during each conversion and a 20^3 state took 19 copies and 19
+// kernels. To and from page-locked memory, FP64: 256^3 download 47.6 -> 45.0 ms
+// (56.6 GB/s, the bus's rate), upload 48.9 -> 46.3; 64^3 1.01 -> 0.75, 1.05 ->
+// 0.77; 20^3 0.228 -> 0.044, 0.230 -> 0.044, and padded, up, two steps and down,
+// 0.571 -> 0.136.) The chunk: large enough to hide a copy's setup (about 10
+// us), small enough that the first conversion, which nothing hides, is short;
+// a slice that goes to several arrays counts by its share of one.
+template <class KERNEL, class COPY>
+static int stream_slices(lbm_solver *s, size_t slice, long long count, bool upload, int arrays,
+    KERNEL &&kernel, COPY &&copy)
+{
+  int rc = need_staging(s, slice);
+  if (rc)
+    return rc;
+  const size_t total = slice * (size_t)count, half = s->staging_bytes / 2 / 256 * 256;
+  const size_t small = (size_t)arrays << 21, least = (size_t)arrays << 22;
+  const size_t most = (size_t)32 << 20;
+  size_t n = count, buffers = 1;
+  if (total > small || total > s->staging_bytes) {
+    n = std::min(half, std::max(least, std::min(most, total / 8))) / slice;
+    buffers = n ? 2 : 1;
+    n = n ? n : 1;
+  }
+  n = std::min(n, (size_t)65535); // grid.z
+  const long long chunks = (count + (long long)n - 1) / (long long)n;
+  char *dev[2] = { (char *)s->staging, (char *)s->staging + (buffers > 1 ? half : 0) };
+  cudaStream_t bus = s->stream;
+  const bool overlap = buffers > 1 && chunks > 1;
+  if (overlap) {
+    for (int b = 0; b < 2; ++b) {
+      if (!s->bus_ev[b])
+        CUDA_TRY(cudaEventCreateWithFlags(&s->bus_ev[b], cudaEventDisableTiming));
+      if (!s->conv_ev[b])
+        CUDA_TRY(cudaEventCreateWithFlags(&s->conv_ev[b], cudaEventDisableTiming));
+    }
+    if (!s->bus)
+      CUDA_TRY(cudaStreamCreateWithFlags(&s->bus, cudaStreamNonBlocking));
+    bus = s->bus;
+    if (upload) { // the staging buffer may be in use by earlier work
+      CUDA_TRY(cudaEventRecord(s->conv_ev[0], s->stream));
+      CUDA_TRY(cudaStreamWaitEvent(bus, s->conv_ev[0], 0));
+    }
+  }
+  for (long long k = 0; k < chunks; ++k) {
+    const int b = (int)(k & 1);
+    const long long i0 = k * (long long)n, m = std::min((long long)n, count - i0);
+    if (overlap && k >= 2) // the buffer's previous chunk has left it
+      CUDA_TRY(cudaStreamWaitEvent(upload ? bus : s->stream,
+          upload ? s->conv_ev[b] : s->bus_ev[b], 0));
+    if (upload) {
+      CUDA_TRY(copy(i0, m, dev[b], bus));
+      if (overlap) {
+        CUDA_TRY(cudaEventRecord(s->bus_ev[b], bus));
+        CUDA_TRY(cudaStreamWaitEvent(s->stream, s->bus_ev[b], 0));
+      }
+    }
+    kernel(i0, m, dev[b]);
+    CUDA_TRY(cudaGetLastError());
+    if (overlap)
+      CUDA_TRY(cudaEventRecord(s->conv_ev[b], s->stream));
+    if (!upload) {
+      if (overlap)
+        CUDA_TRY(cudaStreamWaitEvent(bus, s->conv_ev[b], 0));
+      CUDA_TRY(copy(i0, m, dev[b], bus));
+      if (overlap)
+        CUDA_TRY(cudaEventRecord(s->bus_ev[b], bus));
+    }
+  }
+  if (overlap && !upload)
+    for (int b = 0; b < 2; ++b) // later work may use the staging buffer
+      CUDA_TRY(cudaStreamWaitEvent(s->stream, s->bus_ev[b], 0));
+  return LBM_OK;
+}
+
+// stream_slices to its end: whatever it enqueued has left the caller's memory
+// when this returns, on an error too.
+template <class KERNEL, class COPY>
+static int move_slices(lbm_solver *s, size_t slice, long long count, bool upload, int arrays,
+    KERNEL &&kernel, COPY &&copy)
+{
+  const int rc = stream_slices(s, slice, count, upload, arrays, kernel, copy);
+  if (!rc)
+    return sync_and_check(s);
+  if (s->bus)
+    cudaStreamSynchronize(s->bus);
+  cudaStreamSynchronize(s->stream);
+  return rc;
+}
+
+// A contiguous host array of slices.
+static int move_array(lbm_solver *s, void *host, size_t slice, long long count, bool upload,
+    void (*launch)(lbm_solver *, int, int, void *, int), int arg)
+{
+  char *h = (char *)host;
+  return move_slices(
+      s, slice, count, upload, 1,
+      [&](long long i0, long long n, char *dev) { launch(s, (int)i0, (int)n, dev, arg); },
+      [&](long long i0, long long n, char *dev, cudaStream_t st) {
+        char *p = h + (size_t)i0 * slice;
+        return upload ? cudaMemcpyAsync(dev, p, (size_t)n * slice, cudaMemcpyHostToDevice, st)
+                      : cudaMemcpyAsync(p, dev, (size_t)n * slice, cudaMemcpyDeviceToHost, st);
+      });
+}
+
+template <class ST, bool UP>
+static void launch_dense_slices(lbm_solver *s, int i0, int n, void *dev, int)
 {
   dim3 grid, block;
   user_launch_shape(s, grid, block);
-  const int o = orientation(s);
-  const size_t plane_host = (size_t)s->nx * s->ny * s->nz;
-  using Sx = typename ST::S;
-  Sx *state = (Sx *)state_ptr(s);
-  for (int d = 0; d < Q; ++d) {
-    CUDA_TRY(cudaMemcpyAsync(s->staging, f + d * plane_host, sizeof(double) * plane_host,
-        cudaMemcpyHostToDevice, s->stream));
-    pack_plane_kernel<ST><<<grid, block, 0, s->stream>>>(s->g, s->ub, d, o, s->staging, state,
-        s->mask,
-        (float)(s->precision == LBM_F16 ? s->fp16_scale : 1.0), weight(d));
-    CUDA_TRY(cudaGetLastError());
-  }
-  return sync_and_check(s);
+  grid.z = n;
+  const double sc = s->precision == LBM_F16 ? s->fp16_scale : 1.0;
+  dense_slices_kernel<ST, UP><<<grid, block, 0, s->stream>>>(s->g, s->ub, i0, orientation(s),
+      (double *)dev, (typename ST::S *)state_ptr(s), s->mask, (float)(UP ? sc : 1.0 / sc));
+}
+
+template <class ST> static int pack_all(lbm_solver *s, const double *f)
+{
+  return move_array(s, const_cast<double *>(f), sizeof(double) * (size_t)s->ny * s->nz,
+      (long long)Q * s->nx, true, launch_dense_slices<ST, true>, 0);
 }
 
 template <class ST> static int unpack_all(lbm_solver *s, double *f)
 {
-  dim3 grid, block;
-  user_launch_shape(s, grid, block);
-  const int o = orientation(s);
-  const size_t plane_host = (size_t)s->nx * s->ny * s->nz;
-  using Sx = typename ST::S;
-  const Sx *state = (const Sx *)state_ptr(s);
-  for (int d = 0; d < Q; ++d) {
-    unpack_plane_kernel<ST><<<grid, block, 0, s->stream>>>(s->g, s->ub, d, o, s->staging, state,
-        s->mask, (float)(s->precision == LBM_F16 ? 1.0 / s->fp16_scale : 1.0), weight(d));
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(f + d * plane_host, s->staging, sizeof(double) * plane_host,
-        cudaMemcpyDeviceToHost, s->stream));
-  }
-  return sync_and_check(s);
+  return move_array(s, f, sizeof(double) * (size_t)s->ny * s->nz, (long long)Q * s->nx, false,
+      launch_dense_slices<ST, false>, 0);
 }
 
 extern "C" int lbm_set_state(lbm_solver *s, const double *f)
@@ -1212,76 +1342,58 @@ extern "C" int lbm_load_state(lbm_solver *s, const char *path)
 // Transfers in the reference's own padded layout (for the drop-in kernels)
 // ---------------------------------------------------------------------------
 
-// Slot of f_d(x) in the reference's padded SoA array, relative to one
-// direction plane (indexSoA, src/lbm.h:113-116, ghost offset 1): push and
-// AA odd/initial states keep f_d(x) at (x, d), pull at (x - c_d, d), AA
-// after an even iteration at (x - c_d, inv d) (src/lbm.c:193-294). For a
-// padded plane p the kernel handles direction d = p, or inv p in the AA
-// even orientation.
-__device__ __forceinline__ long long ref_index(int rx, int ry, int rz, int ref_orient, int d,
-    int x, int y, int z)
+// The padded SoA array of the reference (indexSoA, src/lbm.h:113-116, ghost
+// offset 1): push and AA odd/initial states keep f_d(x) at (x, d), pull at
+// (x - c_d, d), AA after an even iteration at (x - c_d, inv d)
+// (src/lbm.c:193-294). Slices i0 .. i0 + gridDim.z - 1 of it, one padded x plane
+// of one direction plane each, sit in `chunk`; each thread takes one padded
+// slot and maps it back to the fluid cell whose population it holds. On
+// download slots that hold none are written as 0.
+template <class ST, typename H, bool UP>
+__global__ void ref_slices_kernel(Grid g, UserBox u, int i0, int ref_orient, int orient,
+    H *__restrict__ chunk, typename ST::S *state, const uint32_t *__restrict__ mask, float scale)
 {
-  int a = x + 1, b = y + 1, c = z + 1;
+  using V = typename ST::V;
+  const int rz = u.nz + 2, ry = u.ny + 2, rx = u.nx + 2;
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = blockIdx.y * blockDim.y + threadIdx.y;
+  const int i = i0 + (int)blockIdx.z;
+  const int p = i / rx, a = i - p * rx;
+  if (c >= rz || b >= ry)
+    return;
+  H *value = chunk + ((long long)blockIdx.z * ry + b) * rz + c;
+  const int d = (ref_orient == LBM_REF_AA_EVEN) ? inv(p) : p;
+  int x = a - 1, y = b - 1, z = c - 1;
   if (ref_orient != LBM_REF_NATURAL) {
-    a -= cx(d);
-    b -= cy(d);
-    c -= cz(d);
+    x += cx(d);
+    y += cy(d);
+    z += cz(d);
   }
-  return ((long long)a * ry + b) * rz + c;
-}
-
-template <class ST, typename H>
-__global__ void pack_ref_kernel(Grid g, UserBox u, int p, int ref_orient, int orient,
-    const H *__restrict__ plane, typename ST::S *state, const uint32_t *__restrict__ mask,
-    float scale)
-{
-  using V = typename ST::V;
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int x = blockIdx.z;
-  if (z >= u.nz || y >= u.ny)
+  bool own = x >= 0 && x < u.nx && y >= 0 && y < u.ny && z >= 0 && z < u.nz;
+  uint32_t cell = 0, m = kSolidBit;
+  if (own)
+    own = locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m);
+  if (!own) {
+    if (!UP)
+      *value = (H)0;
     return;
-  uint32_t cell, m;
-  if (!locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m))
-    return;
-  const int d = (ref_orient == LBM_REF_AA_EVEN) ? inv(p) : p;
+  }
   const Nbr nb = make_nbr(g, x + u.ox, y + u.oy, z + u.oz, cell);
   int sp;
   uint32_t sc;
   state_slot(orient, d, m, cell, nb, sp, sc);
-  double v = (double)plane[ref_index(u.nx + 2, u.ny + 2, u.nz + 2, ref_orient, d, x, y, z)];
-  if (ST::kShifted) {
-    const int wc = wclass(d);
-    v -= wc == 0 ? 1.0 / 3.0 : wc == 1 ? 1.0 / 18.0 : 1.0 / 36.0;
+  typename ST::S *slot = state + (long long)sp * g.plane + sc;
+  if (UP) {
+    double v = (double)*value;
+    if (ST::kShifted)
+      v -= weight_of(d);
+    ST::store(slot, (V)v, (V)scale);
+  } else {
+    double v = (double)ST::load(slot, d, (V)scale);
+    if (ST::kShifted)
+      v += weight_of(d);
+    *value = (H)v;
   }
-  ST::store(state + (long long)sp * g.plane + sc, (V)v, (V)scale);
-}
-
-template <class ST, typename H>
-__global__ void unpack_ref_kernel(Grid g, UserBox u, int p, int ref_orient, int orient,
-    H *__restrict__ plane, const typename ST::S *state, const uint32_t *__restrict__ mask,
-    float inv_scale)
-{
-  using V = typename ST::V;
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int x = blockIdx.z;
-  if (z >= u.nz || y >= u.ny)
-    return;
-  uint32_t cell, m;
-  if (!locate(g, mask, x + u.ox, y + u.oy, z + u.oz, cell, m))
-    return;
-  const int d = (ref_orient == LBM_REF_AA_EVEN) ? inv(p) : p;
-  const Nbr nb = make_nbr(g, x + u.ox, y + u.oy, z + u.oz, cell);
-  int sp;
-  uint32_t sc;
-  state_slot(orient, d, m, cell, nb, sp, sc);
-  double v = (double)ST::load(state + (long long)sp * g.plane + sc, d, (V)inv_scale);
-  if (ST::kShifted) {
-    const int wc = wclass(d);
-    v += wc == 0 ? 1.0 / 3.0 : wc == 1 ? 1.0 / 18.0 : 1.0 / 36.0;
-  }
-  plane[ref_index(u.nx + 2, u.ny + 2, u.nz + 2, ref_orient, d, x, y, z)] = (H)v;
 }
 
 // The same transfer for the reference's AoS array (indexAoS,
@@ -1383,45 +1495,24 @@ static int ref_transfer_aos(lbm_solver *s, void *host, int ref_orient, bool uplo
   return sync_and_check(s);
 }
 
+template <class ST, typename H, bool UP>
+static void launch_ref_slices(lbm_solver *s, int i0, int n, void *dev, int ref_orient)
+{
+  const dim3 block(32, 4, 1);
+  const dim3 grid((s->nz + 2 + 31) / 32, (s->ny + 2 + 3) / 4, n);
+  const float sc = (float)(s->precision == LBM_F16 ? s->fp16_scale : 1.0);
+  ref_slices_kernel<ST, H, UP><<<grid, block, 0, s->stream>>>(s->g, s->ub, i0, ref_orient,
+      orientation(s), (H *)dev, (typename ST::S *)state_ptr(s), s->mask, UP ? sc : 1.0f / sc);
+}
+
 template <class ST, typename H>
 static int ref_transfer(lbm_solver *s, void *host, int ref_orient, bool upload)
 {
   if (ref_orient & LBM_REF_AOS)
     return ref_transfer_aos<ST, H>(s, host, ref_orient & ~LBM_REF_AOS, upload);
-  const size_t gpl = (size_t)(s->nx + 2) * (s->ny + 2) * (s->nz + 2);
-  const size_t bytes = gpl * sizeof(H);
-  if (s->pstaging_bytes < bytes) {
-    cudaFree(s->pstaging);
-    s->pstaging = NULL;
-    s->pstaging_bytes = 0;
-    int rc = dev_alloc(s, &s->pstaging, bytes, "the padded transfer plane");
-    if (rc)
-      return rc;
-    s->pstaging_bytes = bytes;
-  }
-  dim3 grid, block;
-  user_launch_shape(s, grid, block);
-  const int o = orientation(s);
-  const float sc = (float)(s->precision == LBM_F16 ? s->fp16_scale : 1.0);
-  using Sx = typename ST::S;
-  H *hp = (H *)host;
-  H *dp = (H *)s->pstaging;
-  for (int p = 0; p < Q; ++p) {
-    if (upload) {
-      CUDA_TRY(cudaMemcpyAsync(dp, hp + p * gpl, bytes, cudaMemcpyHostToDevice, s->stream));
-      pack_ref_kernel<ST, H><<<grid, block, 0, s->stream>>>(s->g, s->ub, p, ref_orient, o, dp,
-          (Sx *)state_ptr(s), s->mask, sc);
-      CUDA_TRY(cudaGetLastError());
-    } else {
-      // slots that hold no fluid population come back as 0
-      CUDA_TRY(cudaMemsetAsync(dp, 0, bytes, s->stream));
-      unpack_ref_kernel<ST, H><<<grid, block, 0, s->stream>>>(s->g, s->ub, p, ref_orient, o, dp,
-          (const Sx *)state_ptr(s), s->mask, 1.0f / sc);
-      CUDA_TRY(cudaGetLastError());
-      CUDA_TRY(cudaMemcpyAsync(hp + p * gpl, dp, bytes, cudaMemcpyDeviceToHost, s->stream));
-    }
-  }
-  return sync_and_check(s);
+  return move_array(s, host, (size_t)(s->ny + 2) * (s->nz + 2) * sizeof(H),
+      (long long)Q * (s->nx + 2), upload,
+      upload ? launch_ref_slices<ST, H, true> : launch_ref_slices<ST, H, false>, ref_orient);
 }
 
 static int ref_dispatch(lbm_solver *s, void *host, int elem_size, int ref_orient, bool upload)
@@ -1841,20 +1932,32 @@ extern "C" int lbm_time_launches(lbm_solver *s, int steps, double *ms_sum, int *
 
 template <class ST> static int moments_t(lbm_solver *s, double *q[4])
 {
-  dim3 grid, block;
-  user_launch_shape(s, grid, block);
-  const size_t n = (size_t)s->nx * s->ny * s->nz;
+  const size_t plane = (size_t)s->ny * s->nz;
   const float inv = (float)(s->precision == LBM_F16 ? 1.0 / s->fp16_scale : 1.0);
-  for (int k = 0; k < 4; ++k) {
-    if (!q[k])
-      continue;
-    moments_kernel<ST><<<grid, block, 0, s->stream>>>(s->g, s->ub, orientation(s), k,
-        (const typename ST::S *)state_ptr(s), s->mask, inv, s->staging);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaMemcpyAsync(q[k], s->staging, sizeof(double) * n, cudaMemcpyDeviceToHost,
-        s->stream));
-  }
-  return sync_and_check(s);
+  // a slice is one x plane of all four quantities; a chunk of n keeps them in
+  // four arrays of n planes
+  return move_slices(
+      s, 4 * sizeof(double) * plane, s->nx, false, 4,
+      [&](long long x0, long long n, char *dev) {
+        dim3 grid, block;
+        user_launch_shape(s, grid, block);
+        grid.z = (unsigned)n;
+        moments_kernel<ST><<<grid, block, 0, s->stream>>>(s->g, s->ub, (int)x0, orientation(s),
+            (const typename ST::S *)state_ptr(s), s->mask, inv, (double *)dev,
+            (long long)(n * plane));
+      },
+      [&](long long x0, long long n, char *dev, cudaStream_t st) {
+        const size_t bytes = sizeof(double) * (size_t)n * plane;
+        for (int k = 0; k < 4; ++k) {
+          if (!q[k])
+            continue;
+          cudaError_t e = cudaMemcpyAsync(q[k] + (size_t)x0 * plane, dev + k * bytes, bytes,
+              cudaMemcpyDeviceToHost, st);
+          if (e != cudaSuccess)
+            return e;
+        }
+        return cudaSuccess;
+      });
 }
 
 extern "C" int lbm_moments(lbm_solver *s, double *rho, double *ux, double *uy, double *uz)
