@@ -13,6 +13,8 @@
 #include "lbm_sweep.cuh"
 #include "lbm_step_x2.cuh"
 
+extern "C" void lbm_map_pages(void *p, size_t bytes); // host/lbm_host.c
+
 namespace lbm {
 
 enum Precision { kF64 = 0, kF32 = 1, kF16 = 2 };

@@ -836,10 +836,10 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     TRY(dev_alloc(s, &s->buf[1], s->state_bytes, "the second population lattice"));
   TRY(dev_alloc(s, (void **)&s->mask, (size_t)s->g.plane * 4, "the link masks"));
   {
-    // one dense plane, or a whole small (padded) state up to 64 MB
+    // one dense plane; two chunks of stream_slices, or a small (padded) state
     const size_t all = sizeof(double) * Q * (size_t)(nx + 2) * (ny + 2) * (nz + 2);
-    s->staging_bytes = std::max(sizeof(double) * (size_t)nx * ny * nz,
-        std::min(all, (size_t)64 << 20));
+    const size_t chunk = std::max((size_t)4 << 20, std::min((size_t)32 << 20, all / 8));
+    s->staging_bytes = std::max(sizeof(double) * (size_t)nx * ny * nz, std::min(all, 2 * chunk));
     TRY(dev_alloc(s, (void **)&s->staging, s->staging_bytes, "the transfer staging"));
   }
   TRY(dev_alloc(s, (void **)&s->red, sizeof(double) * kRedVals * (kRedBlocks + 1),
@@ -1190,6 +1190,20 @@ static int move_array(lbm_solver *s, void *host, size_t slice, long long count, 
       });
 }
 
+// Before a download into the caller's array: maps its pages unless it is
+// small, page-locked or mapped already.
+static void map_target(void *host, size_t bytes)
+{
+  if (!host || bytes < ((size_t)1 << 20))
+    return;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess)
+    cudaGetLastError(); // not known to CUDA: pageable
+  else if (at.type != cudaMemoryTypeUnregistered)
+    return;
+  lbm_map_pages(host, bytes);
+}
+
 template <class ST, bool UP>
 static void launch_dense_slices(lbm_solver *s, int i0, int n, void *dev, int)
 {
@@ -1209,6 +1223,7 @@ template <class ST> static int pack_all(lbm_solver *s, const double *f)
 
 template <class ST> static int unpack_all(lbm_solver *s, double *f)
 {
+  map_target(f, sizeof(double) * Q * (size_t)s->nx * s->ny * s->nz);
   return move_array(s, f, sizeof(double) * (size_t)s->ny * s->nz, (long long)Q * s->nx, false,
       launch_dense_slices<ST, false>, 0);
 }
@@ -1934,6 +1949,8 @@ template <class ST> static int moments_t(lbm_solver *s, double *q[4])
 {
   const size_t plane = (size_t)s->ny * s->nz;
   const float inv = (float)(s->precision == LBM_F16 ? 1.0 / s->fp16_scale : 1.0);
+  for (int k = 0; k < 4; ++k)
+    map_target(q[k], sizeof(double) * s->nx * plane);
   // a slice is one x plane of all four quantities; a chunk of n keeps them in
   // four arrays of n planes
   return move_slices(
