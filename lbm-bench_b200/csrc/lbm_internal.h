@@ -50,6 +50,7 @@ struct SweepLaunch {
   void *f; // the lattice
   const uint32_t *mask;
   const float *porosity; // Brinkman term, or NULL
+  void *u_save;          // momenta of the sweep's steps (Brinkman only), or NULL
   SweepPlan p;
   bool force, flip;
 };

@@ -76,6 +76,8 @@ struct lbm_solver {
   int no_shuffle; // reduced precision: never use the shuffle-aligned kernels
   int no_quad;    // FP16 AA: never use the four-cell kernels
   void *u_save_next; // adjoint recomputation: momentum output of the next step
+  void *adj_ws;      // adjoint workspace kept between gradients, or NULL
+  size_t adj_bytes;
   int slab;          // x-slab of a decomposed domain: device planes 0 and nx+1 are ghosts
   int tma;           // FP64 steps use the bulk-copy pipelined kernels (shape in tma_shape)
   int tma_groups;    // consumer groups of 8 warps per CTA
@@ -554,6 +556,7 @@ static void free_all(lbm_solver *s)
   cudaFree(s->cwb);
   delete s->cplane0;
   cudaFree(s->sweep_done);
+  cudaFree(s->adj_ws);
   free(s->split_done);
   if (s->fork_ev)
     cudaEventDestroy(s->fork_ev);
@@ -1814,8 +1817,9 @@ extern "C" int lbm_set_pressure_bc(lbm_solver *s, double rho_in, double rho_out,
   return LBM_OK;
 }
 
-// Launches a sweep of `steps` steps (even, at most s->sweep_steps).
-static int launch_sweep(lbm_solver *s, int steps)
+// Launches a sweep of `steps` steps (even, at most s->sweep_steps); u_save as
+// in SweepArgsD.
+static int launch_sweep(lbm_solver *s, int steps, void *u_save = NULL)
 {
   SweepLaunch l;
   l.g = s->g;
@@ -1827,6 +1831,7 @@ static int launch_sweep(lbm_solver *s, int steps)
     l.p.blocks = l.p.front * (uint32_t)s->g.nx * (uint32_t)(steps / 2);
   const bool brink = s->alpha != 0.0 && s->porosity;
   l.porosity = brink ? s->porosity : NULL;
+  l.u_save = brink ? u_save : NULL;
   l.force = s->force_on || brink;
   l.flip = s->pattern == LBM_PULL;
   CUDA_TRY(cudaMemsetAsync(s->sweep_done, 0,
@@ -2467,6 +2472,27 @@ __global__ void grad_to_dense_kernel(Grid g, UserBox u, const double *__restrict
   dense[dense_index(u, x, y, z)] = (mask[cell] & kSolidBit) ? 0.0 : grad[cell];
 }
 
+// Largest adjoint workspace a solver keeps between gradients: 2% of the device.
+constexpr size_t kKeptWorkspace = (size_t)4 << 30;
+
+// Runs `len` Brinkman steps, saving the momentum of step i at ub + i * ubytes.
+static int run_saving(lbm_solver *s, int len, char *ub, size_t ubytes)
+{
+  int rc = LBM_OK;
+  for (int i = 0; i < len && !rc;) {
+    if (const int n = next_sweep(s, len - i)) {
+      rc = launch_sweep(s, n, ub + (size_t)i * ubytes);
+      i += n;
+      continue;
+    }
+    s->u_save_next = ub + (size_t)i * ubytes;
+    rc = launch_one(s, NULL);
+    s->u_save_next = NULL;
+    ++i;
+  }
+  return rc;
+}
+
 extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_every,
     double *grad, double *j_out, double *info)
 {
@@ -2504,7 +2530,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
   if (k == LBM_CKPT_AUTO) {
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    const double budget = 0.9 * (double)free_b;
+    const double budget = 0.9 * (double)(free_b + s->adj_bytes);
     k = std::min(k_sqrt, steps);
     // memory grows with k beyond k_sqrt; the largest fitting k by bisection
     long long lo = k, hi = steps;
@@ -2533,10 +2559,20 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
 #define ATRY(x)                                                                               do {                                                                                          cudaError_t err_ = (x);                                                                     if (err_ != cudaSuccess) {                                                                    rc = fail(err_ == cudaErrorMemoryAllocation ? LBM_ERR_ALLOC : LBM_ERR_CUDA,                    "lbm_adjoint_gradient: %s: %s", #x, cudaGetErrorString(err_));                         goto done;                                                                                }                                                                                         } while (0)
 #define RTRY(x)                                                                               do {                                                                                          rc = (x);                                                                                   if (rc)                                                                                       goto done;                                                                              } while (0)
   {
-    ATRY(cudaMalloc((void **)&ck, (size_t)nck * s->state_bytes));
-    ATRY(cudaMalloc((void **)&ub, (size_t)k * ubytes));
-    ATRY(cudaMalloc((void **)&lam, 2 * lbytes));
-    ATRY(cudaMalloc((void **)&dg, P * 8));
+    // one workspace, kept for the solver's next gradient when it is small
+    // (allocating and freeing it took 3-4 of 20 ms at 96^3 x 100 steps)
+    if (s->adj_bytes < extra) {
+      cudaFree(s->adj_ws);
+      s->adj_ws = NULL;
+      s->dev_bytes -= s->adj_bytes;
+      s->adj_bytes = 0;
+      RTRY(dev_alloc(s, &s->adj_ws, extra, "the adjoint workspace"));
+      s->adj_bytes = extra;
+    }
+    dg = (double *)s->adj_ws; // each part is a multiple of the plane's 256 bytes
+    lam = (char *)(dg + P);
+    ck = lam + 2 * lbytes;
+    ub = ck + (size_t)nck * s->state_bytes;
     ATRY(cudaEventCreate(&e0));
     ATRY(cudaEventCreate(&e1));
     const long long t0 = s->steps_done;
@@ -2553,13 +2589,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
         RTRY(lbm_run(s, len));
         continue;
       }
-      for (int i = 0; i < len; ++i) {
-        s->u_save_next = ub + (size_t)i * ubytes;
-        rc = launch_one(s, NULL);
-        s->u_save_next = NULL;
-        if (rc)
-          goto done;
-      }
+      RTRY(run_saving(s, len, ub, ubytes));
     }
     ATRY(cudaEventRecord(e1, s->stream));
     ATRY(cudaEventSynchronize(e1));
@@ -2584,13 +2614,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
         ATRY(cudaMemcpyAsync(state, ck + (size_t)c * s->state_bytes, s->state_bytes,
             cudaMemcpyDeviceToDevice, s->stream));
         s->steps_done = t0 + tc;
-      }
-      for (int i = 0; i < len && c < nck - 1; ++i) {
-        s->u_save_next = ub + (size_t)i * ubytes;
-        rc = launch_one(s, NULL);
-        s->u_save_next = NULL;
-        if (rc)
-          goto done;
+        RTRY(run_saving(s, len, ub, ubytes));
       }
       for (int i = len - 1; i >= 0; --i) {
         if (f64) {
@@ -2651,15 +2675,17 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
       info[2] = k;
       info[3] = nck;
       info[4] = (double)extra;
-      info[5] = (double)(s->dev_bytes + extra);
+      info[5] = (double)(s->dev_bytes - s->adj_bytes + extra);
     }
   }
 done:
   s->u_save_next = NULL;
-  cudaFree(ck);
-  cudaFree(ub);
-  cudaFree(lam);
-  cudaFree(dg);
+  if (s->adj_bytes > kKeptWorkspace || rc) {
+    cudaFree(s->adj_ws); // waits for what uses it
+    s->adj_ws = NULL;
+    s->dev_bytes -= s->adj_bytes;
+    s->adj_bytes = 0;
+  }
   if (e0)
     cudaEventDestroy(e0);
   if (e1)

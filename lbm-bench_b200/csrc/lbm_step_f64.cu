@@ -253,6 +253,7 @@ static cudaError_t pick_sweep(const SweepLaunch &l, const Consts<double> &c, cud
   a.c = c;
   a.p = l.p;
   a.porosity = l.porosity;
+  a.u_save = (double *)l.u_save;
   const bool fronts = l.p.lag > 0;
   if (!l.g.wb) {
     if constexpr (FORCE && !FLIP)

@@ -181,6 +181,7 @@ static cudaError_t pick_sweep(const SweepLaunch &l, const Consts2 &c, cudaStream
   a.c = c;
   a.p = l.p;
   a.porosity = l.porosity;
+  a.u_save = (float *)l.u_save;
   if (!l.g.wb) {
     const bool fronts = l.p.lag > 0;
     if constexpr (FORCE && !FLIP)

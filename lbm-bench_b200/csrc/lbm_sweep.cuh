@@ -301,10 +301,12 @@ struct SweepCp {
 #endif
 
 // FP64, dense layout, one cell per thread (step_kernel). BRINK adds the
-// Brinkman term of a.porosity. Offsets of the 19 planes fit 32 bits (checked
+// Brinkman term of a.porosity, and saves each step's momentum (3 planes a step,
+// u_save from the sweep's first step on) when u_save is set. Offsets of the 19 planes fit 32 bits (checked
 // at planning).
 template <class ST> struct SweepArgsD : SweepArgs<ST> {
   const float *porosity;
+  typename ST::V *u_save;
 };
 
 template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct SweepDense {
@@ -371,8 +373,15 @@ template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct Sweep
     if (BRINK)
       kappa = a.c.alpha * (V(1.0) - V(a.porosity[cell]));
     V o[Q];
-    collide<V, BRINK>(v, o, a.c, kappa);
+    V u3[3];
+    collide<V, BRINK>(v, o, a.c, kappa, BRINK ? u3 : nullptr);
     cell = recompute(cell);
+    if (BRINK && a.u_save) {
+      V *u = a.u_save + 3 * (long long)it.s * g.plane + cell;
+      u[0] = u3[0];
+      u[g.plane] = u3[1];
+      u[2 * g.plane] = u3[2];
+    }
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const bool bb = (mask >> d) & 1u;

@@ -197,6 +197,7 @@ struct SweepCp2 {
 // bits (checked at planning).
 template <class ST> struct SweepArgsD2 : SweepArgs2<ST> {
   const float *porosity;
+  float *u_save; // as in SweepArgsD
 };
 
 template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct SweepDense2 {
@@ -252,9 +253,15 @@ template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct Sweep
       const float2 por = *reinterpret_cast<const float2 *>(a.porosity + cell);
       kappa = make_float2(a.c.alpha * (1.f - por.x), a.c.alpha * (1.f - por.y));
     }
-    float2 o[Q];
-    collide2<BRINK>(f, o, a.c, kappa, nullptr);
+    float2 o[Q], u3[3];
+    collide2<BRINK>(f, o, a.c, kappa, BRINK ? u3 : nullptr);
     cell = recompute(cell);
+    if (BRINK && a.u_save) {
+      float *u = a.u_save + 3 * (long long)it.s * g.plane + cell;
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        *reinterpret_cast<float2 *>(u + k * g.plane) = u3[k];
+    }
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       // a wall cell's own slot is never read: both cells are written
@@ -310,9 +317,19 @@ template <class ST, bool FORCE, bool FLIP, bool BRINK, bool FRONTS> struct Sweep
     if (BRINK)
       kappa = make_float2(fl0 ? a.c.alpha * (1.f - a.porosity[cell]) : 0.f,
           fl1 ? a.c.alpha * (1.f - a.porosity[cell + 32u]) : 0.f);
-    float2 o[Q];
-    collide2<BRINK>(f, o, a.c, kappa, nullptr);
+    float2 o[Q], u3[3];
+    collide2<BRINK>(f, o, a.c, kappa, BRINK ? u3 : nullptr);
     cell = recompute(cell);
+    if (BRINK && a.u_save) {
+      float *u = a.u_save + 3 * (long long)it.s * g.plane + cell;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (fl0)
+          u[k * g.plane] = u3[k].x;
+        if (fl1)
+          u[k * g.plane + 32] = u3[k].y;
+      }
+    }
 #pragma unroll
     for (int d = 0; d < Q; ++d) {
       const float2 v = FORCE ? add_force2(o[d], d, m0, m1, a.c.force) : o[d];

@@ -81,3 +81,21 @@ def test_brinkman_sweeps_equal_single_steps(pattern, dims, precision):
                 s.run(n)
             out.append(s.get_state())
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [L.F64, L.F32])
+@pytest.mark.parametrize("dims", [(24, 30, 41), (81, 131, 141)])
+def test_gradient_does_not_depend_on_sweeps(dims, precision):
+    """checkpoint_every = 1 recomputes single steps; longer segments sweep
+    (even and odd lengths), saving each step's momentum."""
+    por = np.random.default_rng(4).uniform(0, 1, dims).astype(np.float32)
+    out = []
+    for k in (1, 4, 5, 11):
+        with _solver(dims, "porous", "aa", precision, False) as s:
+            s.set_porosity(por, 0.1)
+            out.append(s.adjoint_gradient(11, k)[:2])
+            again = s.adjoint_gradient(11, k)[:2]  # in the kept workspace
+            assert again[0] == out[-1][0] and np.array_equal(again[1], out[-1][1])
+    for j, g in out[1:]:
+        assert j == out[0][0] and np.array_equal(g, out[0][1])
