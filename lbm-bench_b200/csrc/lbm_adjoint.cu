@@ -1,4 +1,5 @@
-// Adjoint kernels (lbm_adjoint.cuh), instantiated for FP64 and FP32.
+// Adjoint kernels (lbm_adjoint.cuh): the FP32 step and the seeds. The FP64
+// steps are in lbm_step_f64.cu.
 #include "lbm_adjoint.cuh"
 #include "lbm_internal.h"
 
@@ -22,10 +23,6 @@ static cudaError_t seed(const Grid &g, int xo, double inv_count, void *lam,
   return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_step_f64(const AdjArgs<double> &a, cudaStream_t st)
-{
-  return step(a, st);
-}
 cudaError_t launch_adjoint_step_f32(const AdjArgs<float> &a, cudaStream_t st)
 {
   return step(a, st);

@@ -69,6 +69,9 @@ cudaError_t launch_pressure_bc(int precision, const Grid &g, const UserBox &u, i
 // the final state for the outlet objective on device plane x = xo.
 cudaError_t launch_adjoint_step_f64(const AdjArgs<double> &a, cudaStream_t st);
 cudaError_t launch_adjoint_step_f32(const AdjArgs<float> &a, cudaStream_t st);
+// A sweep of reverse steps in a.lam, in place; a.u: the latest step's momentum.
+cudaError_t launch_adjoint_sweep_f64(const AdjArgs<double> &a, const SweepPlan &p,
+    cudaStream_t st);
 cudaError_t launch_adjoint_seed(int precision, const Grid &g, int xo, double inv_count,
     void *lam, const uint32_t *mask, cudaStream_t st);
 

@@ -2493,6 +2493,53 @@ static int run_saving(lbm_solver *s, int len, char *ub, size_t ubytes)
   return rc;
 }
 
+template <typename V>
+static AdjArgs<V> adj_args(const lbm_solver *s, const void *from, void *to, const void *u,
+    double *grad)
+{
+  AdjArgs<V> a;
+  a.g = s->g;
+  a.lam_next = (const V *)from;
+  a.lam = (V *)to;
+  a.u = (const V *)u;
+  a.mask = s->mask;
+  a.porosity = s->porosity;
+  a.grad = grad;
+  a.oE = (V)s->omega;
+  a.oO = (V)(1.0 / (0.5 + s->lambda / (1.0 / s->omega - 0.5)));
+  a.w0 = (V)(1.0 / 3.0);
+  a.w1 = (V)(1.0 / 18.0);
+  a.w2 = (V)(1.0 / 36.0);
+  a.alpha = (V)s->alpha;
+  return a;
+}
+
+// Plan of the FP64 reverse steps' sweeps: one cell per thread, shifted step
+// first. plan.steps = 0 where forward steps do not sweep either.
+static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
+{
+  SweepPlan p;
+  p.steps = 0;
+  if (!s->sweep_steps || s->precision != LBM_F64)
+    return p;
+  SweepShape h;
+  h.nx = s->g.nx;
+  h.ny = s->g.ny;
+  h.units = (uint32_t)((s->g.nz + 31) / 32);
+  h.row_start = NULL;
+  h.pair = false;
+  h.local_first = false;
+  h.plane_bytes = (double)s->state_bytes / s->g.nx;
+  h.resident = 8u * (uint32_t)sm_count();
+  const bool fronts = s->state_bytes > 60e6;
+  if (!sweep_plan(h, fronts, p))
+    p.steps = 0;
+  else
+    p.steps = fronts ? 2 : kSweepMaxSteps;
+  p.err = s->dev_err;
+  return p;
+}
+
 extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_every,
     double *grad, double *j_out, double *info)
 {
@@ -2550,7 +2597,11 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
   if (k > steps)
     k = steps;
   const int nck = (steps + k - 1) / k;
-  const size_t extra = (size_t)nck * s->state_bytes + (size_t)k * ubytes + 2 * lbytes + P * 8;
+  SweepPlan plan = plan_adjoint_sweep(s);
+  const size_t counters = plan.steps
+      ? sizeof(uint32_t) * sweep_counter(plan, s->g.nx, plan.steps - 1, 0, 0) : 0;
+  const size_t extra = (size_t)nck * s->state_bytes + (size_t)k * ubytes + 2 * lbytes + P * 8 +
+      counters;
 
   char *ck = NULL, *ub = NULL, *lam = NULL;
   double *dg = NULL;
@@ -2573,6 +2624,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
     lam = (char *)(dg + P);
     ck = lam + 2 * lbytes;
     ub = ck + (size_t)nck * s->state_bytes;
+    plan.done = (uint32_t *)(ub + (size_t)k * ubytes);
     ATRY(cudaEventCreate(&e0));
     ATRY(cudaEventCreate(&e1));
     const long long t0 = s->steps_done;
@@ -2616,41 +2668,26 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
         s->steps_done = t0 + tc;
         RTRY(run_saving(s, len, ub, ubytes));
       }
-      for (int i = len - 1; i >= 0; --i) {
-        if (f64) {
-          AdjArgs<double> a;
-          a.g = s->g;
-          a.lam_next = (const double *)(lam + cur * lbytes);
-          a.lam = (double *)(lam + (cur ^ 1) * lbytes);
-          a.u = (const double *)(ub + (size_t)i * ubytes);
-          a.mask = s->mask;
-          a.porosity = s->porosity;
-          a.grad = dg;
-          a.oE = s->omega;
-          a.oO = 1.0 / (0.5 + s->lambda / (1.0 / s->omega - 0.5));
-          a.w0 = 1.0 / 3.0;
-          a.w1 = 1.0 / 18.0;
-          a.w2 = 1.0 / 36.0;
-          a.alpha = s->alpha;
-          ATRY(launch_adjoint_step_f64(a, s->stream));
-        } else {
-          AdjArgs<float> a;
-          a.g = s->g;
-          a.lam_next = (const float *)(lam + cur * lbytes);
-          a.lam = (float *)(lam + (cur ^ 1) * lbytes);
-          a.u = (const float *)(ub + (size_t)i * ubytes);
-          a.mask = s->mask;
-          a.porosity = s->porosity;
-          a.grad = dg;
-          a.oE = (float)s->omega;
-          a.oO = (float)(1.0 / (0.5 + s->lambda / (1.0 / s->omega - 0.5)));
-          a.w0 = (float)(1.0 / 3.0);
-          a.w1 = (float)(1.0 / 18.0);
-          a.w2 = (float)(1.0 / 36.0);
-          a.alpha = (float)s->alpha;
-          ATRY(launch_adjoint_step_f32(a, s->stream));
+      // steps len - 1 .. 0, in sweeps as far as there are pairs
+      for (int i = len - 1; i >= 0;) {
+        const char *u = ub + (size_t)i * ubytes;
+        char *from = lam + cur * lbytes, *to = lam + (cur ^ 1) * lbytes;
+        const int n = std::min((i + 1) & ~1, plan.steps);
+        if (n) {
+          SweepPlan p = plan;
+          p.steps = n;
+          p.blocks = (p.lag ? p.slab_blocks * p.slabs : p.front * (uint32_t)s->g.nx * (n / 2));
+          ATRY(cudaMemsetAsync(p.done, 0,
+              sizeof(uint32_t) * sweep_counter(p, s->g.nx, n - 1, 0, 0), s->stream));
+          s->err_pending = 1;
+          ATRY(launch_adjoint_sweep_f64(adj_args<double>(s, from, from, u, dg), p, s->stream));
+          i -= n;
+          continue;
         }
+        ATRY(f64 ? launch_adjoint_step_f64(adj_args<double>(s, from, to, u, dg), s->stream)
+                 : launch_adjoint_step_f32(adj_args<float>(s, from, to, u, dg), s->stream));
         cur ^= 1;
+        --i;
       }
     }
     ATRY(cudaEventRecord(e1, s->stream));

@@ -282,4 +282,26 @@ cudaError_t launch_sweep_f64(const SweepLaunch &l, const Consts<double> &c, cuda
   return l.force ? pick_sweep<true, false>(l, c, st) : pick_sweep<false, false>(l, c, st);
 }
 
+// FP64 reverse steps. Without contraction a step and a sweep compile to the
+// same operations, so a gradient does not depend on which of them ran a step
+// (with it, the last bits did; FP32 steps are contracted and do not sweep).
+cudaError_t launch_adjoint_step_f64(const AdjArgs<double> &a, cudaStream_t st)
+{
+  dim3 grid, block;
+  cell_launch_shape(a.g, grid, block);
+  adjoint_step_kernel<double><<<grid, block, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_sweep_f64(const AdjArgs<double> &a, const SweepPlan &p, cudaStream_t st)
+{
+  SweepAdjArgs<double> q;
+  static_cast<AdjArgs<double> &>(q) = a;
+  q.src = a.lam;
+  q.dst = a.lam;
+  q.p = p;
+  return p.lag ? go_sweep<SweepAdjoint<double, true>>(q, st)
+               : go_sweep<SweepAdjoint<double, false>>(q, st);
+}
+
 } // namespace lbm
