@@ -1067,19 +1067,29 @@ static void user_launch_shape(const lbm_solver *s, dim3 &grid, dim3 &block)
   cell_launch_shape(gu, grid, block);
 }
 
-// At least `bytes` of device staging.
+// At least `bytes` of device staging. A buffer that cannot grow stays as it is:
+// other calls need no more than they had.
 static int need_staging(lbm_solver *s, size_t bytes)
 {
   if (s->staging_bytes >= bytes)
     return LBM_OK;
+  const size_t had = s->staging_bytes;
   CUDA_TRY(cudaStreamSynchronize(s->stream));
-  cudaFree(s->staging);
-  s->staging = NULL;
-  s->dev_bytes -= s->staging_bytes;
-  s->staging_bytes = 0;
-  int rc = dev_alloc(s, (void **)&s->staging, bytes, "the transfer staging");
-  if (!rc)
-    s->staging_bytes = bytes;
+  void *p = NULL;
+  int rc = dev_alloc(s, &p, bytes, "the transfer staging");
+  if (!rc || had) {
+    cudaFree(s->staging);
+    s->staging = (double *)p;
+    s->staging_bytes = rc ? 0 : bytes;
+    s->dev_bytes -= had;
+  }
+  if (rc && had) { // in the old buffer's place, or the old buffer again
+    rc = dev_alloc(s, (void **)&s->staging, bytes, "the transfer staging");
+    if (!rc)
+      s->staging_bytes = bytes;
+    else if (!dev_alloc(s, (void **)&s->staging, had, "the transfer staging"))
+      s->staging_bytes = had;
+  }
   return rc;
 }
 
@@ -2698,6 +2708,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
     ATRY(cudaMemcpyAsync(state, ck, s->state_bytes, cudaMemcpyDeviceToDevice, s->stream));
     s->steps_done = t0;
     {
+      RTRY(need_staging(s, sizeof(double) * (size_t)s->nx * s->ny * s->nz));
       dim3 grid, block;
       user_launch_shape(s, grid, block);
       grad_to_dense_kernel<<<grid, block, 0, s->stream>>>(s->g, s->ub, dg, s->mask, s->staging);

@@ -1,0 +1,63 @@
+"""Host paths of the solver without a GPU: the library's own objects linked
+with a CUDA runtime that counts launches and limits memory (fake_cudart.cpp)."""
+import ctypes
+import glob
+import importlib.util
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+import lbmb200
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "lbm-bench_b200")
+
+
+@pytest.fixture(scope="module")
+def L(tmp_path_factory):
+    """The binding over the fake runtime, with .fake (the library)."""
+    subprocess.run(["make", "-C", PKG, "-j8"], check=True, capture_output=True)
+    objs = [o for o in sorted(glob.glob(os.path.join(PKG, "_build", "lbm_*.o")))
+            if not o.endswith("_sp.o")]
+    so = tmp_path_factory.mktemp("fake") / "libfake.so"
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-I/usr/local/cuda/include",
+                    os.path.join(ROOT, "tests", "fake_cudart.cpp"), *objs, "-o", str(so),
+                    "-Wl,-Bsymbolic", "-fopenmp", "-ldl"], check=True, capture_output=True)
+    spec = importlib.util.spec_from_file_location("lbmb200_fake", lbmb200.__file__)
+    mod = importlib.util.module_from_spec(spec)
+    sys.modules["lbmb200_fake"] = mod
+    spec.loader.exec_module(mod)
+    mod.LIB_PATH = str(so)
+    mod.fake = mod.lib()
+    mod.fake.fake_limit.argtypes = [ctypes.c_size_t]
+    mod.fake.fake_used.restype = ctypes.c_size_t
+    mod.fake.fake_launches.restype = ctypes.c_long
+    yield mod
+    mod.fake.fake_limit(1 << 40)
+
+
+def _porous_solver(L, dims, precision=None):
+    flags = np.ones(dims[::-1], np.int32)
+    s = L.Solver(flags, (1, 1, 1), "aa", L.F64 if precision is None else precision)
+    s.set_porosity(np.full(dims, 0.5, np.float32), 0.1)
+    return s
+
+
+def test_failed_staging_growth_leaves_the_solver_usable(L):
+    """A slice of the moments of 1 x 1500 x 1500 (72 MB) is larger than the
+    staging the solver was created with: growing it fails, and the gradient's
+    download, which needs no more than before, still has its buffer."""
+    with _porous_solver(L, (1, 1500, 1500)) as s:
+        s.adjoint_gradient(2, 1)
+        before = s.device_bytes
+        L.fake.fake_limit(L.fake.fake_used() + (1 << 20))
+        with pytest.raises(L.LbmError):
+            s.moments()
+        L.fake.fake_limit(1 << 40)
+        s.adjoint_gradient(2, 1)
+        assert s.device_bytes == before
+        s.moments()
+        assert s.device_bytes > before
