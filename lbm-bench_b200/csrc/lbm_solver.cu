@@ -668,8 +668,8 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
   int rc = dev_alloc(s, (void **)&s->sweep_done,
       sizeof(uint32_t) * sweep_counter(s->sweep, s->g.nx, steps - 1, 0, 0),
       "the sweep counters");
-  if (rc)
-    return rc;
+  if (rc) // a full device: single steps
+    return rc == LBM_ERR_ALLOC ? LBM_OK : rc;
   s->sweep.done = s->sweep_done;
   s->sweep.err = s->dev_err;
   s->sweep_steps = steps;
@@ -838,13 +838,6 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
   if (pattern != LBM_AA)
     TRY(dev_alloc(s, &s->buf[1], s->state_bytes, "the second population lattice"));
   TRY(dev_alloc(s, (void **)&s->mask, (size_t)s->g.plane * 4, "the link masks"));
-  {
-    // one dense plane; two chunks of stream_slices, or a small (padded) state
-    const size_t all = sizeof(double) * Q * (size_t)(nx + 2) * (ny + 2) * (nz + 2);
-    const size_t chunk = std::max((size_t)4 << 20, std::min((size_t)32 << 20, all / 8));
-    s->staging_bytes = std::max(sizeof(double) * (size_t)nx * ny * nz, std::min(all, 2 * chunk));
-    TRY(dev_alloc(s, (void **)&s->staging, s->staging_bytes, "the transfer staging"));
-  }
   TRY(dev_alloc(s, (void **)&s->red, sizeof(double) * kRedVals * (kRedBlocks + 1),
       "reduction partials"));
   TRYC(cudaMemsetAsync(s->buf[0], 0, s->state_bytes, s->stream));
@@ -878,8 +871,6 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
       s->tma_shape.blocks = s->tma_shape.ntiles < sms ? s->tma_shape.ntiles : sms;
     }
   }
-
-  TRY(init_sweep(s, row_start));
 
   {
     // cells of the Zou-He pressure boundary (src/lbm.c:693-700): flag 2 on
@@ -955,6 +946,21 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     std::vector<uint32_t> pad((size_t)(s->g.plane - cells), kSolidBit);
     TRYC(cudaMemcpy(s->mask + cells, pad.data(), pad.size() * 4, cudaMemcpyHostToDevice));
   }
+  // last, so that what it can do without (chunked staging, the sweeps'
+  // counters) takes no memory from the rest
+  {
+    // one dense plane; two chunks of stream_slices, or a small (padded) state,
+    // where there is room for them
+    const size_t all = sizeof(double) * Q * (size_t)(nx + 2) * (ny + 2) * (nz + 2);
+    const size_t chunk = std::max((size_t)4 << 20, std::min((size_t)32 << 20, all / 8));
+    const size_t least = sizeof(double) * (size_t)nx * ny * nz;
+    s->staging_bytes = std::max(least, std::min(all, 2 * chunk));
+    if (dev_alloc(s, (void **)&s->staging, s->staging_bytes, "the transfer staging")) {
+      s->staging_bytes = least;
+      TRY(dev_alloc(s, (void **)&s->staging, least, "the transfer staging"));
+    }
+  }
+  TRY(init_sweep(s, row_start));
 #undef TRY
 #undef TRYC
   *out = s;

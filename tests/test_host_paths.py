@@ -61,3 +61,39 @@ def test_failed_staging_growth_leaves_the_solver_usable(L):
         assert s.device_bytes == before
         s.moments()
         assert s.device_bytes > before
+
+
+@pytest.mark.parametrize("compact", [False, True])
+def test_creation_needs_no_memory_for_what_it_can_do_without(L, compact):
+    """On a nearly full device a solver is created without the sweeps'
+    counters and with staging for one dense plane, and takes single steps."""
+    dims = (512, 16, 32)
+    flags = np.ones(dims[::-1], np.int32)
+    cells = 512 * 16 * 32
+
+    def make():
+        return L.Solver(flags, (1, 1, 1), "aa", L.F64, compact=compact)
+
+    with make() as s:
+        s.run(8)
+        assert s.launch_count == 1
+        full = s.device_bytes
+        assert full == L.fake.fake_used()
+    # state, link masks, staging plane, the build's fluid bytes; compact: the
+    # index and the build's dense masks; 64 KB of reduction partials and padding
+    least = 19 * 8 * cells + 4 * cells + 8 * cells + cells + (1 << 16)
+    if compact:
+        least += 8 * cells // 32 + 4 * cells
+    assert least < full
+    try:
+        for limit in range(least, full + 1, (full - least) // 16):
+            L.fake.fake_limit(limit)
+            with make() as s:
+                s.run(8)
+                assert s.steps_done == 8
+                assert s.launch_count == 8 or limit > least
+                s.get_state()
+                s.moments()
+    finally:
+        L.fake.fake_limit(1 << 40)
+    assert L.fake.fake_used() == 0
