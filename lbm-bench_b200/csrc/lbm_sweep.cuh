@@ -183,6 +183,67 @@ __device__ __forceinline__ void sweep_prefetch(const Grid &g, const S *src,
     l2_prefetch_bytes(mask, lo * 4ull, hi * 4ull);
 }
 
+// RowTab for a sweep's shifted step. Where z wraps, RowTab::at looks each of the
+// ten neighbours above and below up when it is asked, one after the other, and
+// a sweep asks twice, behind its wait: sweeps of z-periodic boxes were slower
+// than single steps (256^3 without walls, us a step, single / lookups / this
+// table: FP64 pull 803 / 909 / 612, AA 852 / 709 / 630, FP32 pull 461 / 523 /
+// 312; FP64 AA 32^3 5.1 / 5.8 / 3.3). Here they are six more entries of the table:
+// the first cell of a row is stored at the row's start and the last one before
+// the next row's start, and those words are loaded together before the wait.
+template <bool ZPER> struct SweepTab : RowTab<ZPER> {
+  using T = RowTab<ZPER>;
+  static constexpr int kRows = kTabRows + (ZPER ? 6 : 0);
+
+  // entry of row q's z - 1 (the index is one less); 4, the own row
+  __device__ __forceinline__ static int below(int q)
+  {
+    return kTabRows + (q == 1 ? 0 : q == 3 ? 1 : q == 5 ? 2 : q == 7 ? 3 : 4);
+  }
+  static constexpr int kOwnAbove = kTabRows + 5;
+
+  __device__ __forceinline__ void build(const Grid &g, int x, int y, int z, uint32_t cell,
+      uint32_t wi, uint32_t lt, int lane, uint32_t k0)
+  {
+    T::template build<true>(g, x, y, z, cell, wi, lt, lane, k0);
+    if constexpr (ZPER) {
+      const bool first = z == 0, last = z == g.nz - 1;
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int q = i < 4 ? 2 * i + 1 : 4;
+        int xr = x + q / 3 - 1, yr = y + q % 3 - 1;
+        xr = xr < 0 ? g.nx - 1 : xr >= g.nx ? 0 : xr;
+        yr = yr < 0 ? g.ny - 1 : yr >= g.ny ? 0 : yr;
+        const uint32_t row = (uint32_t)xr * (uint32_t)g.ny + (uint32_t)yr;
+        const int up = q == 4 ? kOwnAbove : T::axis_slot(q);
+        uint32_t lo = T::B[q], hi = q == 4 ? cell + 1u : T::B[up];
+        if (first)
+          lo = __ldg(&g.wb[(row + 1u) * (uint32_t)g.W].y);
+        if (last)
+          hi = __ldg(&g.wb[row * (uint32_t)g.W].y);
+        T::sB[below(q) * kStepThreads] = lo;
+        T::sB[up * kStepThreads] = hi;
+        if (q != 4)
+          T::B[up] = hi;
+      }
+    }
+  }
+
+  __device__ __forceinline__ uint32_t at(const Grid &g, int d, bool regs = false) const
+  {
+    if constexpr (ZPER) {
+      const int q = (cx(d) + 1) * 3 + (cy(d) + 1);
+      if (cz(d) < 0)
+        return T::sB[below(q) * kStepThreads] - 1u;
+      if (cz(d) > 0)
+        return q == 4 ? T::sB[kOwnAbove * kStepThreads] : T::entry(T::axis_slot(q), regs);
+      return T::entry(q, regs);
+    } else {
+      return T::at(g, d, regs);
+    }
+  }
+};
+
 template <class ST> struct SweepArgs {
   Grid g;
   const typename ST::S *src; // the lattice, twice: with one pointer the compiler keeps
@@ -244,12 +305,12 @@ struct SweepCp {
   __device__ __forceinline__ static void shifted(const Args &a, const SweepItem &it, int tid,
       WAIT &&wait)
   {
-    __shared__ uint32_t tab[kTabRows * kStepThreads];
+    __shared__ uint32_t tab[SweepTab<ZPER>::kRows * kStepThreads];
     const Grid &g = a.g;
     const int lane = tid & 31;
     int y;
     uint32_t wi;
-    RowTab<ZPER> t;
+    SweepTab<ZPER> t;
     t.sB = tab + tid;
     bool fluid = false;
     uint32_t cell = 0, mask = 0;
@@ -260,7 +321,7 @@ struct SweepCp {
       fluid = (wb0.x >> lane) & 1u;
       cell = wb0.y + (uint32_t)__popc(wb0.x & lt);
       mask = __ldg(a.mask + (fluid ? cell : 0u));
-      t.template build<true>(g, it.x, y, (int)(32u * wi) + lane, cell, wi, lt, lane, k0);
+      t.build(g, it.x, y, (int)(32u * wi) + lane, cell, wi, lt, lane, k0);
     }
     wait();
     if (!fluid)

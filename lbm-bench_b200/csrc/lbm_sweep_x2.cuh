@@ -115,14 +115,14 @@ struct SweepCp2 {
   __device__ __forceinline__ static void shifted(const Args &a, const SweepItem &it, int tid,
       WAIT &&wait)
   {
-    __shared__ uint32_t tab[2 * kTabRows * kStepThreads];
+    __shared__ uint32_t tab[2 * SweepTab<ZPER>::kRows * kStepThreads];
     const Grid &g = a.g;
     const int lane = tid & 31;
     int y;
     uint32_t unit;
-    RowTab<ZPER> t0, t1;
+    SweepTab<ZPER> t0, t1;
     t0.sB = tab + tid;
-    t1.sB = tab + kTabRows * kStepThreads + tid;
+    t1.sB = tab + SweepTab<ZPER>::kRows * kStepThreads + tid;
     bool fl0 = false, fl1 = false;
     uint32_t cell0 = 0, cell1 = 0, m0 = 0, m1 = 0;
     if (sweep_unit(a.p, g.ny, it, tid >> 5, y, unit)) {
@@ -139,9 +139,9 @@ struct SweepCp2 {
       m0 = fl0 ? __ldg(a.mask + cell0) : 0u;
       m1 = fl1 ? __ldg(a.mask + cell1) : 0u;
       const int z0 = 32 * (int)wi0 + lane;
-      t0.template build<true>(g, it.x, y, z0, cell0, wi0, lt, lane, k0);
+      t0.build(g, it.x, y, z0, cell0, wi0, lt, lane, k0);
       if (has1)
-        t1.template build<true>(g, it.x, y, z0 + 32, cell1, wi0 + 1u, lt, lane, k0 + 1u);
+        t1.build(g, it.x, y, z0 + 32, cell1, wi0 + 1u, lt, lane, k0 + 1u);
     }
     wait();
     if (!fl0 && !fl1)

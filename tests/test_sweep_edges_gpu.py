@@ -1,0 +1,37 @@
+"""Sweeps against single steps, bit for bit, at edges that test_sweep.py's boxes
+do not have: run(n) sweeps, n calls of run(1) do not."""
+import numpy as np
+import pytest
+
+import lbmb200 as L
+
+pytestmark = pytest.mark.gpu
+
+
+def _states(flags, per, pattern, precision, compact, runs, force=True, porosity=None):
+    """State after each list of runs, and the launches it took."""
+    out = []
+    for steps in runs:
+        with L.Solver(flags, per, pattern, precision, compact=compact) as s:
+            s.set_params(1.3, 3 / 16, 1e-5, force)
+            if porosity is not None:
+                s.set_porosity(porosity, 0.1)
+            s.init_equilibrium(seed=5, amplitude=1e-3)
+            for n in steps:
+                s.run(n)
+            out.append((s.get_state(), s.launch_count))
+    return out
+
+
+@pytest.mark.parametrize("pattern", ["aa", "pull", "push"])
+@pytest.mark.parametrize("precision", [L.F64, L.F32, L.F16])
+@pytest.mark.parametrize("dims", [(70, 90, 1), (60, 60, 2), (16, 20, 31), (16, 20, 32),
+                                  (16, 20, 33), (12, 20, 64), (12, 20, 65), (8, 20, 96)])
+def test_rows_that_wrap_in_z(dims, precision, pattern):
+    """Compact layout, periodic z: first and last cells of rows of one cell, of
+    part of a word, of whole words and of one cell more, with walls on them."""
+    flags = (np.random.default_rng(sum(dims)).uniform(size=dims[::-1]) > 0.3).astype(np.int32)
+    (ref, singles), (got, launches) = _states(flags, (1, 1, 1), pattern, precision, True,
+                                              ((1,) * 8, (8,)))
+    assert singles == 8 and launches == 1
+    assert np.array_equal(got, ref)
