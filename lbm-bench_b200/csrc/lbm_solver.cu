@@ -617,9 +617,9 @@ static int sync_and_check(lbm_solver *s)
 // C ABI
 // ---------------------------------------------------------------------------
 
-// Whether, and in which order, a solver runs sweeps, and their plan. The
-// lines (lattice bytes) lie where one order or single steps begin to win; us
-// per step, single steps / step-major / fronts, channels of 64 x 64 planes on a
+// Whether, and in which order, a solver runs sweeps (sweep_pays), and their
+// plan. Step-major up to 85 MB, where its order begins to lose to fronts; us per
+// step, single steps / step-major / fronts, channels of 64 x 64 planes on a
 // B200:
 //   compact FP64 AA    43 MB 12.4 / 9.6 / 14.9   65 MB 16.6 / 14.3 / 19.6
 //                      87 MB 25.8 / 24.6 / 24.3   108 MB 39.0 / 37.2 / 29.7
@@ -636,21 +636,18 @@ static int sync_and_check(lbm_solver *s)
 //   dense FP16 AA      65 MB 44.1 / 33.1 / 36.9   97 MB 69.0 / 54.5 / 53.9
 //   dense FP16 pull    65 MB 36.9 / 34.4 / 36.4   97 MB 53.0 / 55.8 / 52.3
 // and at 256^3 (20% solid) in ms, single / fronts: compact FP16 AA 0.274 /
-// 0.305, pull 0.316 / 0.304, push 0.356 / 0.305; dense FP16 pull 0.302 / 0.321
-// (its single steps read rows of whole 64-cell segments in aligned pairs).
-// Below 4096 cells (16^3) nothing was measured.
+// 0.305 (single steps above 33 MB), pull 0.316 / 0.304, push 0.356 / 0.305;
+// dense FP16 pull 0.302 / 0.321. Below 4096 cells (16^3) nothing was measured.
 static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
 {
-  if (s->slab || s->tma || s->n_fluid < 4096)
+  if (s->slab || s->tma || s->n_fluid < 4096 || sm_count() == 0)
     return LBM_OK;
   // the dense layout's sweeps address the 19 planes with 32-bit offsets
   if (!s->compact && (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return LBM_OK;
   const double mb = s->state_bytes / 1e6;
   const bool fronts = mb > 85.0;
-  if (s->precision == LBM_F16 &&
-      (s->compact ? s->pattern == LBM_AA && mb > 33.0
-                  : s->pattern == LBM_PULL && fronts && s->g.nz % 64 == 0))
+  if (s->precision == LBM_F16 && s->compact && s->pattern == LBM_AA && mb > 33.0)
     return LBM_OK;
   SweepShape h;
   h.nx = s->g.nx;
@@ -663,6 +660,14 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
   h.plane_bytes = (double)s->state_bytes / s->g.nx;
   h.resident = 8u * (uint32_t)sm_count(); // all sweep kernels run 7 or 8 blocks per SM
   if (!sweep_plan(h, fronts, s->sweep))
+    return LBM_OK;
+  SweepUse u = sweep_use(h, s->sweep, (double)s->n_fluid);
+  u.bytes = (int)storage_size(s->precision);
+  u.aa = s->pattern == LBM_AA;
+  u.zper = (s->g.per & 4) != 0;
+  u.nz = s->g.nz;
+  u.fluid = (double)s->n_fluid / ((double)s->g.nx * s->g.ny * s->g.nz);
+  if (!sweep_pays(u, fronts))
     return LBM_OK;
   const int steps = fronts ? 2 : kSweepMaxSteps;
   int rc = dev_alloc(s, (void **)&s->sweep_done,
@@ -2531,12 +2536,19 @@ static AdjArgs<V> adj_args(const lbm_solver *s, const void *from, void *to, cons
 }
 
 // Plan of the FP64 reverse steps' sweeps: one cell per thread, shifted step
-// first. plan.steps = 0 where forward steps do not sweep either.
+// first; plan.steps = 0 for single steps. 60 steps' reverse sweep with its
+// recomputation, single / sweep, ms: channels 64^3 (40 MB) 1.65 / 1.13, 96 x
+// 64^2 (60 MB) 2.67 / 1.76 step-major, 128 x 64^2 (80 MB) 3.75 / 2.81, 160^3
+// 25.9 / 18.8 in fronts. Below a third of a block's cells in use, or in a
+// mostly solid box, empty blocks cost more than HBM (16384 x 6^2, 0.06: 11.1 /
+// 12.1; pipe in 300 x 300 x 16: 2.22 / 4.70; 300^2 x 16, 0.43: 12.8 / 10.9).
 static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
 {
   SweepPlan p;
   p.steps = 0;
-  if (!s->sweep_steps || s->precision != LBM_F64)
+  if (s->precision != LBM_F64 || s->slab || s->tma || s->compact || s->n_fluid < 4096 ||
+      s->g.nx < 4 || sm_count() == 0 ||
+      (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return p;
   SweepShape h;
   h.nx = s->g.nx;
@@ -2548,7 +2560,10 @@ static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
   h.plane_bytes = (double)s->state_bytes / s->g.nx;
   h.resident = 8u * (uint32_t)sm_count();
   const bool fronts = s->state_bytes > 60e6;
-  if (!sweep_plan(h, fronts, p))
+  const bool ok = sweep_plan(h, fronts, p);
+  const SweepUse u = sweep_use(h, p, (double)s->n_fluid);
+  const double fluid = (double)s->n_fluid / ((double)s->g.nx * s->g.ny * s->g.nz);
+  if (!ok || (u.waves > 3.1 && (u.fill < 0.33 || (fronts && fluid < 0.25))))
     p.steps = 0;
   else
     p.steps = fronts ? 2 : kSweepMaxSteps;

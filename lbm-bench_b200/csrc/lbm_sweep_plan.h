@@ -198,4 +198,94 @@ inline bool sweep_plan(const SweepShape &h, bool fronts, SweepPlan &p)
       ((uint64_t)h.ny * h.units + kSweepWarps) * h.units < (1ull << 32);
 }
 
+// Where a sweep is faster than single steps. A block of a sweep costs a wait
+// and a release besides its cells; single steps pack cells of several planes
+// into a block and have kernels for special cases that sweeps do not have
+// (rows without links, rows of whole 64-cell segments).
+struct SweepUse {
+  int bytes;     // of a stored population
+  bool aa, pull; // else push
+  bool compact, zper;
+  int nx, nz;
+  double mb;     // lattice
+  double fluid;  // fluid share of the box
+  double plane_cells; // fluid cells of a plane, on average
+  double fill;   // fluid cells per cell that the blocks of a step could take
+  double waves;  // blocks of a step, in blocks that run at a time
+};
+
+inline SweepUse sweep_use(const SweepShape &h, const SweepPlan &p, double cells)
+{
+  SweepUse u = SweepUse();
+  const double blocks = 0.5 * p.front * p.slabs * h.nx;
+  u.nx = h.nx;
+  u.compact = h.row_start != nullptr;
+  u.pull = !h.local_first;
+  u.mb = h.plane_bytes * h.nx / 1e6;
+  u.plane_cells = cells / h.nx;
+  u.fill = cells / (blocks * kSweepThreads * (h.pair ? 2 : 1));
+  u.waves = blocks / h.resident;
+  return u;
+}
+
+// Measured on a B200 at about 250 boxes (fully periodic, channels, pipes,
+// blocks and spheres; 1 to 65535 planes) in every pattern, precision and
+// layout; us per step, single steps / sweep, (fill).
+inline bool sweep_pays(const SweepUse &u, bool fronts)
+{
+  const bool pair = u.bytes < 8, push = !u.aa && !u.pull;
+  // few planes: each waits for nearly the whole step before
+  if (u.nx < 4 && u.waves > 0.2) {
+    if (u.compact) { // channel 2 x 300^2, FP64 AA 9.2 / 11.1; periodic 1 x 512^2, push 18.4 / 11.9,
+      if (!u.zper || (u.pull && (fronts || !pair))) // pull 2 x 1000^2 102 / 109
+        return false;
+    } else if (!pair ? u.waves > 0.5 : u.bytes == 4 ? fronts && !u.aa : u.pull || u.waves > 3.1) {
+      return false; // FP64 pull 2 x 300^2 9.3 / 11.9; FP32 pull 2 x 1000^2 51.7 / 56.7, AA 64.6 /
+    }               // 52.4; FP16 pull 1 x 512^2 6.2 / 8.6
+  }
+  // thin planes and mostly solid boxes: blocks with few cells
+  if (u.compact && u.zper) // FP32 push 16384 x 3^2 51.2 / 68.3, 4096 x 4^2 19.5 / 15.8; FP64 AA
+    // 16384 x 3^2 44.1 / 49.8, 4096 x 8^2 30.7 / 22.7; pull in a fifth of 256 x 128^2 57.4 / 71.9
+    return u.waves <= (pair ? 2.0 : 3.0) || (u.fluid >= 0.25 && u.plane_cells >= 16);
+  if (u.compact) {
+    if (u.waves <= (pair ? 2.0 : 3.0)) // 64^3 channel, FP64 AA 11.3 / 8.3, FP16 push 9.2 / 5.2
+      return true;
+    if (push) // FP16 channels: 2048 x 32^2 50.1 / 58.8 (half of each pair of words is
+      return pair ? u.nz > 32 && u.fill >= 0.25 : u.fill >= 0.1; // missing), 1024 x 40^2 57.4 / 41.5
+    if (u.pull) // FP64 pull pipe in 369 x 287 x 32 28.2 / 28.9 (0.14), 71^2 x 297 22.6 / 19.8 (0.28)
+      return u.fill >= (u.bytes == 2 ? 0.15 : 0.2);
+    if (u.bytes == 2) // 300^2 x 8 59.5 / 65.0 (0.17), pipe in 184 x 73 x 98 25.0 / 24.7 (0.58)
+      return u.fill >= 0.4;
+    if (pair && fronts) // 1024 x 40^2 (100 MB) 45.0 / 46.6 (0.62), 128^3 52.6 / 42.4,
+      return u.nx >= 8 && (u.fill >= 0.75 || u.mb > 130); // 517 x 75 x 92 (164 MB) 78.5 / 73.2
+    return u.fill >= 0.3; // FP64 AA 8192 x 10^2 45.1 / 57.2 (0.25), 300^2 x 8 55.0 / 53.7 (0.31)
+  }
+  // FP16 single pull steps of rows of whole segments: 128^3 36.9 / 41.7, channel
+  // 41.4 / 43.0; periodic 64-cell rows 300 x 64^2 21.0 / 22.4
+  const bool segments = u.bytes == 2 && u.pull &&
+      (u.nz % 128 == 0 || (u.zper && u.nz % 64 == 0));
+  if (u.waves <= (!segments ? 3.1 : u.nx >= 8 ? 2.0 : 0.2)) // 64^3 channel, FP64 AA 11.3 / 8.0,
+    return true;                                            // FP32 push 10.2 / 5.0
+  // a mostly solid box touches less than the L2 holds (pipe in 369 x 287 x 32:
+  // FP64 AA 23.8 / 55.4, FP32 pull 24.6 / 40.5)
+  if (fronts && u.fluid < 0.25)
+    return false;
+  if (push) // periodic 16384 x 3^2 FP64 41.0 / 49.3 (0.07); 65535 x 2^2 FP32 163 / 204 (0.02)
+    return u.fill >= (!u.zper ? 0.015 : pair ? 0.03 : 0.15);
+  if (u.pull) {
+    if (!pair) // periodic 16384 x 3^2 38.9 / 45.6 (0.07)
+      return u.fill >= (u.zper ? 0.15 : 0.05);
+    if (u.bytes == 2 && (segments || u.nx < 8)) // 4 x 1000^2 76.3 / 84.2
+      return false;
+    // FP32 channel 248 x 329 x 24 82.0 / 85.5 (0.34); pipe in 93 x 378 x 162 82.5 / 68.1 (0.28)
+    return u.fill >= (u.nz > 32 ? 0.25 : u.bytes == 4 || !u.zper ? 0.4 : 0.55);
+  }
+  if (!pair) // 8192 x 8^2 52.7 / 59.1 (0.25); channel 1024 x 24^2 (90 MB) 23.4 / 26.1 (0.63)
+    return u.fill >= (!fronts ? 0.3 : u.mb <= 100 ? 0.7 : 0.26);
+  if (u.bytes == 4) // periodic 8192 x 8^2 62.6 / 65.1 (0.12); channel 8192 x 10^2 118 / 85.7 (0.08)
+    return u.fill >= (u.zper ? 0.2 : 0.015);
+  // FP16 128-cell rows without walls 256^3 272 / 297, with 20% spheres 355 / 310
+  return u.fill >= (u.zper ? 0.03 : 0.015) && !(u.nz % 128 == 0 && u.fluid > 0.9);
+}
+
 } // namespace lbm

@@ -97,3 +97,60 @@ def test_creation_needs_no_memory_for_what_it_can_do_without(L, compact):
     finally:
         L.fake.fake_limit(1 << 40)
     assert L.fake.fake_used() == 0
+
+
+# (box, geometry, pattern, precision, compact, whether run(8) sweeps): boxes at
+# which sweeps measured slower than single steps, each beside one of the same
+# kind at which they are faster
+ROUTES = [
+    ((16384, 3, 3), "fluid", "push", "fp32", True, False),  # thin planes
+    ((4096, 8, 8), "fluid", "push", "fp32", True, True),
+    ((16384, 3, 3), "fluid", "push", "fp64", False, False),
+    ((8192, 10, 10), "channel", "aa", "fp64", True, False),
+    ((2048, 24, 24), "channel", "aa", "fp64", True, True),
+    ((2, 300, 300), "channel", "aa", "fp64", True, False),  # few planes
+    ((2, 300, 300), "fluid", "pull", "fp64", False, False),
+    ((16, 128, 128), "fluid", "pull", "fp64", True, True),
+    ((1024, 24, 24), "channel", "push", "fp16", True, False),  # rows of one word
+    ((1024, 40, 40), "channel", "push", "fp16", True, True),
+    ((200, 200, 33), "pipe", "aa", "fp64", False, False),   # mostly solid box
+    ((200, 100, 33), "channel", "aa", "fp64", False, True),
+    ((128, 128, 128), "fluid", "pull", "fp16", False, False),  # rows of whole segments
+    ((96, 96, 96), "fluid", "pull", "fp16", False, True),
+    ((64, 64, 64), "channel", "aa", "fp64", False, True),
+]
+
+
+@pytest.mark.parametrize("dims,kind,pattern,precision,compact,sweeps", ROUTES)
+def test_sweeps_run_where_they_are_faster(L, dims, kind, pattern, precision, compact, sweeps):
+    flags, per, _ = L.geometry(kind, dims, (1, 0, 0))
+    with L.Solver(flags, per, L.PATTERNS[pattern], L.PRECISIONS[precision], compact=compact) as s:
+        s.run(8)
+        assert s.steps_done == 8
+        assert (s.launch_count < 8) == sweeps
+
+
+def test_counters_stay_small(L):
+    """31 counters of a cache line for each plane of a long thin box would be
+    more memory than its lattice."""
+    for dims in ((60000, 3, 3), (4096, 4, 4), (2900, 3, 3)):
+        flags = np.ones(dims[::-1], np.int32)
+        for compact in (False, True):
+            with L.Solver(flags, (1, 1, 1), "aa", L.F64, compact=compact) as s:
+                s.run(64)
+                state = 19 * 8 * flags.size
+                assert s.device_bytes < 3 * state + (16 << 20)
+
+
+@pytest.mark.parametrize("dims,kind,sweeps", [((16384, 6, 6), "channel", False),
+                                              ((300, 200, 16), "pipe", False),
+                                              ((64, 64, 64), "channel", True),
+                                              ((128, 64, 64), "channel", True)])
+def test_reverse_sweeps_run_where_they_are_faster(L, dims, kind, sweeps):
+    flags, per, _ = L.geometry(kind, dims, (1, 0, 0))
+    with L.Solver(flags, per, "aa", L.F64) as s:
+        s.set_porosity(np.full(dims, 0.5, np.float32), 0.1)
+        L.fake.fake_launches(b"", 1)
+        s.adjoint_gradient(8, 8)
+        assert (L.fake.fake_launches(b"SweepAdjoint", 0) > 0) == sweeps
+        assert (L.fake.fake_launches(b"adjoint_step_kernel", 0) == 8) != sweeps
