@@ -642,8 +642,13 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
 {
   if (s->slab || s->tma || s->n_fluid < 4096 || sm_count() == 0)
     return LBM_OK;
-  // the dense layout's sweeps address the 19 planes with 32-bit offsets
-  if (!s->compact && (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
+  // Sweeps address the 19 planes with 32-bit offsets, but for the compact FP64
+  // layout: 64-bit offsets of two cells per thread do not fit the registers
+  // (channel 640^3, ms a step, single / sweep: FP64 AA 12.9 / 10.8, pull 12.8 / 10.6;
+  // FP32 AA 7.64 / 7.67 with 184-376 bytes of spills, pull 7.8 / 8.8, FP16 pull
+  // 6.2 / 7.3).
+  if ((!s->compact || s->precision != LBM_F64) &&
+      (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return LBM_OK;
   const double mb = s->state_bytes / 1e6;
   const bool fronts = mb > 85.0;

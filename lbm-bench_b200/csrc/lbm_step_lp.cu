@@ -192,15 +192,11 @@ static cudaError_t pick_sweep(const SweepLaunch &l, const Consts2 &c, cudaStream
                   : go_sweep<SweepDense2<ST, FORCE, FLIP, false, false>>(a, st);
   }
   const bool zper = (l.g.per & 4) != 0;
-  const bool off32 = (unsigned long long)Q * (unsigned long long)l.g.plane < (1ull << 32);
-  if (l.p.lag == 0) // the lattice fits the L2, so its offsets fit 32 bits
-    return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, false, uint32_t>>(a, st)
-                : go_sweep<SweepCp2<ST, FORCE, FLIP, false, false, uint32_t>>(a, st);
-  if (off32)
-    return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, true, uint32_t>>(a, st)
-                : go_sweep<SweepCp2<ST, FORCE, FLIP, false, true, uint32_t>>(a, st);
-  return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, true, uint64_t>>(a, st)
-              : go_sweep<SweepCp2<ST, FORCE, FLIP, false, true, uint64_t>>(a, st);
+  if (l.p.lag == 0)
+    return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, false>>(a, st)
+                : go_sweep<SweepCp2<ST, FORCE, FLIP, false, false>>(a, st);
+  return zper ? go_sweep<SweepCp2<ST, FORCE, FLIP, true, true>>(a, st)
+              : go_sweep<SweepCp2<ST, FORCE, FLIP, false, true>>(a, st);
 }
 
 template <class ST>

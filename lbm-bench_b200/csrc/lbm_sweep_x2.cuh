@@ -33,9 +33,9 @@ template <class ST> struct SweepArgs2 {
 #endif
 
 // Compact layout. Local step: two consecutive stored cells per thread.
-// Shifted step: cells z and z + 32 of one row per thread.
-template <class ST, bool FORCE, bool FLIP, bool ZPER, bool FRONTS, typename OFF>
-struct SweepCp2 {
+// Shifted step: cells z and z + 32 of one row per thread. Offsets of the 19
+// planes fit 32 bits (checked at planning).
+template <class ST, bool FORCE, bool FLIP, bool ZPER, bool FRONTS> struct SweepCp2 {
   using Args = SweepArgs2<ST>;
   using PT = PairOf<ST>;
   using S = typename PT::S;
@@ -43,9 +43,9 @@ struct SweepCp2 {
   static constexpr int kMinBlocks = LBM_MINB_SWEEP_CP2;
   static constexpr bool kLocalFirst = !FLIP;
 
-  __device__ static OFF el(const Args &a, int plane, uint32_t i)
+  __device__ static uint32_t el(const Args &a, int plane, uint32_t i)
   {
-    return (OFF)(FLIP ? inv(plane) : plane) * (OFF)a.g.plane + (OFF)i;
+    return (uint32_t)(FLIP ? inv(plane) : plane) * (uint32_t)a.g.plane + i;
   }
 
   // The pair (cell, cell + 1), cell even.
@@ -146,7 +146,7 @@ struct SweepCp2 {
     wait();
     if (!fl0 && !fl1)
       return;
-    auto ld = [&](bool fl, OFF o) { return fl ? PT::dec1(a.src[o]) : 0.0f; };
+    auto ld = [&](bool fl, uint32_t o) { return fl ? PT::dec1(a.src[o]) : 0.0f; };
     float2 f[Q];
     if (!__any_sync(__activemask(), ((m0 | m1) & 0x7FFFFu) != 0u)) {
 #pragma unroll
@@ -157,8 +157,8 @@ struct SweepCp2 {
 #pragma unroll
       for (int d = 0; d < Q; ++d) {
         const bool b0 = (m0 >> inv(d)) & 1u, b1 = (m1 >> inv(d)) & 1u;
-        const OFF o0 = b0 ? el(a, d, cell0) : el(a, inv(d), t0.at(g, inv(d), true));
-        const OFF o1 = b1 ? el(a, d, cell1) : el(a, inv(d), t1.at(g, inv(d), true));
+        const uint32_t o0 = b0 ? el(a, d, cell0) : el(a, inv(d), t0.at(g, inv(d), true));
+        const uint32_t o1 = b1 ? el(a, d, cell1) : el(a, inv(d), t1.at(g, inv(d), true));
         f[d] = make_float2(ld(fl0, o0), ld(fl1, o1));
       }
     }

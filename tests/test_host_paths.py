@@ -154,3 +154,16 @@ def test_reverse_sweeps_run_where_they_are_faster(L, dims, kind, sweeps):
         s.adjoint_gradient(8, 8)
         assert (L.fake.fake_launches(b"SweepAdjoint", 0) > 0) == sweeps
         assert (L.fake.fake_launches(b"adjoint_step_kernel", 0) == 8) != sweeps
+
+
+@pytest.mark.slow
+def test_wide_offsets_sweep_in_fp64_only(L):
+    """Lattices of 2^32 elements and more (here by a few planes) need 64-bit
+    offsets, with which the two-cell sweeps spill and are slower."""
+    dims = (2048, 332, 333)
+    assert 19 * dims[0] * dims[1] * dims[2] >= 2 ** 32
+    flags = np.ones(dims[::-1], np.int32)
+    for precision, sweeps in ((L.F64, True), (L.F32, False)):
+        with L.Solver(flags, (1, 1, 1), "pull", precision, compact=True) as s:
+            s.run(8)
+            assert (s.launch_count < 8) == sweeps

@@ -35,3 +35,30 @@ def test_rows_that_wrap_in_z(dims, precision, pattern):
                                               ((1,) * 8, (8,)))
     assert singles == 8 and launches == 1
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.slow
+@pytest.mark.parametrize("kind", ["fluid", "channel"])
+def test_wide_offsets(kind):
+    """Compact FP64 lattices of more than 2^32 elements, compared on the
+    device: sweeps of AA and pull against single AA steps."""
+    dims = (2048, 336, 336)
+    flags, per, fluid = L.geometry(kind, dims, (1, 0, 0))
+    assert 19 * int((flags != 0).sum()) >= 2 ** 32
+
+    def make(pattern):
+        s = L.Solver(flags, per, pattern, L.F64, compact=True)
+        s.set_params(1.3, 3 / 16, 1e-5, True)
+        s.init_equilibrium(seed=5, amplitude=1e-3)
+        return s
+
+    with make("aa") as ref:
+        for _ in range(4):
+            ref.run(1)
+        assert ref.launch_count == 4
+        for pattern in ("aa", "pull"):
+            with make(pattern) as s:
+                s.run(4)
+                assert s.launch_count == 2
+                out = s.compare(ref)
+                assert out[0] == out[2] == out[4] == 0.0 and out[3] > 0.0
