@@ -97,6 +97,7 @@ struct lbm_solver {
   uint2 *cwb; // compact layout: (fluid bits, first index) per row word
   std::vector<uint32_t> *cplane0; // storage index of the first fluid cell of each x plane (nx+1)
   // sweeps (lbm_sweep.cuh): several steps per launch, planned at creation
+  int no_sweep;         // LBM_B200_NO_SWEEP=1, or a sweep's wait ran out: single steps only
   int sweep_steps;      // most steps of one launch; 0: single steps only
   SweepPlan sweep;
   uint32_t *sweep_done; // its counters
@@ -595,20 +596,25 @@ static int dev_alloc(lbm_solver *s, void **p, size_t bytes, const char *what)
 }
 
 // Waits for the solver's stream, then reports a kernel whose bounded wait ran
-// out since the last check (the error word is copied only if a launch may
-// have set it).
-static int sync_and_check(lbm_solver *s)
+// out since the last check. The error word is copied if a launch since then may
+// have set it, or `always` (also launches that a caller captured and replays).
+// After a sweep's wait ran out the solver takes single steps, which wait for
+// nothing.
+static int sync_and_check(lbm_solver *s, bool always = false)
 {
   unsigned int err = 0;
-  if (s->err_pending)
+  const bool read = s->err_pending || always;
+  if (read)
     CUDA_TRY(cudaMemcpyAsync(&err, s->dev_err, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
   CUDA_TRY(cudaStreamSynchronize(s->stream));
-  if (!s->err_pending)
-    return LBM_OK;
   s->err_pending = 0;
   if (!err)
     return LBM_OK;
-  CUDA_TRY(cudaMemset(s->dev_err, 0, sizeof(err)));
+  if (err & kErrSweepWait) {
+    s->no_sweep = 1;
+    s->sweep_steps = 0;
+  }
+  CUDA_TRY(cudaMemsetAsync(s->dev_err, 0, sizeof(err), s->stream));
   return fail(LBM_ERR_CUDA, "a step kernel gave up waiting for %s; the state is undefined",
       err & kErrBulkCopy ? "its bulk copies" : "the blocks of an earlier step");
 }
@@ -640,7 +646,7 @@ static int sync_and_check(lbm_solver *s)
 // dense FP16 pull 0.302 / 0.321. Below 4096 cells (16^3) nothing was measured.
 static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
 {
-  if (s->slab || s->tma || s->n_fluid < 4096 || sm_count() == 0)
+  if (s->no_sweep || s->slab || s->tma || s->n_fluid < 4096 || sm_count() == 0)
     return LBM_OK;
   // Sweeps address the 19 planes with 32-bit offsets, but for the compact FP64
   // layout: 64-bit offsets of two cells per thread do not fit the registers
@@ -682,6 +688,8 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
     return rc == LBM_ERR_ALLOC ? LBM_OK : rc;
   s->sweep.done = s->sweep_done;
   s->sweep.err = s->dev_err;
+  if (const char *spin = getenv("LBM_B200_SWEEP_SPIN")) // polls before a wait gives up
+    s->sweep.spin = (uint32_t)strtoul(spin, NULL, 10);
   s->sweep_steps = steps;
   return LBM_OK;
 }
@@ -727,6 +735,8 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
     s->no_shuffle = (ns && ns[0] == '1') ? 1 : 0;
     const char *nq = getenv("LBM_B200_NO_QUAD");
     s->no_quad = (nq && nq[0] == '1') ? 1 : 0;
+    const char *nw = getenv("LBM_B200_NO_SWEEP");
+    s->no_sweep = (nw && nw[0] == '1') ? 1 : 0;
   }
   cudaGetDevice(&s->device);
 
@@ -1913,7 +1923,7 @@ extern "C" int lbm_synchronize(lbm_solver *s)
     return fail(LBM_ERR_ARG, "lbm_synchronize: NULL solver");
   if (s->side)
     CUDA_TRY(cudaStreamSynchronize(s->side));
-  return sync_and_check(s);
+  return sync_and_check(s, true);
 }
 
 extern "C" int lbm_run_timed(lbm_solver *s, int steps, double *ms)
@@ -1931,7 +1941,7 @@ extern "C" int lbm_run_timed(lbm_solver *s, int steps, double *ms)
   float t = 0.f;
   CUDA_TRY(cudaEventElapsedTime(&t, s->ev[0], s->ev[1]));
   *ms = t;
-  return sync_and_check(s);
+  return sync_and_check(s, true);
 }
 
 extern "C" int lbm_time_launches(lbm_solver *s, int steps, double *ms_sum, int *count,
@@ -1973,7 +1983,7 @@ extern "C" int lbm_time_launches(lbm_solver *s, int steps, double *ms_sum, int *
     return rc;
   if (e != cudaSuccess)
     return fail(LBM_ERR_CUDA, "lbm_time_launches: %s", cudaGetErrorString(e));
-  return sync_and_check(s);
+  return sync_and_check(s, true);
 }
 
 template <class ST> static int moments_t(lbm_solver *s, double *q[4])
@@ -2551,7 +2561,8 @@ static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
 {
   SweepPlan p;
   p.steps = 0;
-  if (s->precision != LBM_F64 || s->slab || s->tma || s->compact || s->n_fluid < 4096 ||
+  if (s->no_sweep || s->precision != LBM_F64 || s->slab || s->tma || s->compact ||
+      s->n_fluid < 4096 ||
       s->g.nx < 4 || sm_count() == 0 ||
       (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return p;

@@ -26,7 +26,8 @@
 // chained-scan kernels assume), so it is running or done; taking the order
 // from an atomic ticket instead cost 5.7% (0.553 against 0.522 ms a step at
 // 256^3). Every wait has an iteration limit all the same, after which the
-// kernel sets the solver's error word and goes on.
+// kernel sets the solver's error word and goes on (its accesses are in range
+// whatever the order); the host then reports it and keeps to single steps.
 //   fronts (lattice larger than the L2): two steps, the second `lag` planes
 //     behind the first.
 //   step-major (lattice in the L2): all planes of a step, then the next
@@ -44,7 +45,6 @@
 namespace lbm {
 
 static_assert(kSweepThreads == kStepThreads, "block size");
-constexpr uint32_t kSweepSpin = 1u << 20; // wait iterations (about a second)
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p)
 {
@@ -64,7 +64,7 @@ __device__ __forceinline__ void sweep_wait(const SweepPlan &p, int nx, const Swe
   for (uint32_t n = 0;; ++n) {
     if (__all_sync(0xFFFFFFFFu, !need || ld_acquire(c) >= target))
       break;
-    if (n >= kSweepSpin || ((n & 1023u) == 1023u && ld_acquire(p.err) != 0u)) {
+    if (n >= p.spin || ((n & 1023u) == 1023u && ld_acquire(p.err) != 0u)) {
       if (lane == 0)
         atomicOr(p.err, kErrSweepWait);
       break;

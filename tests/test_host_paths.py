@@ -167,3 +167,45 @@ def test_wide_offsets_sweep_in_fp64_only(L):
         with L.Solver(flags, (1, 1, 1), "pull", precision, compact=True) as s:
             s.run(8)
             assert (s.launch_count < 8) == sweeps
+
+
+def test_a_sweep_that_gave_up_leaves_single_steps(L):
+    """The error word set by a sweep's kernel: the next call that waits reports
+    it, and later steps and gradients run as single steps."""
+    with _porous_solver(L, (64, 64, 64)) as s:
+        s.run(8)
+        assert s.launch_count == 1
+        L.fake.fake_raise(2)
+        with pytest.raises(L.LbmError, match="gave up waiting"):
+            s.synchronize()
+        s.synchronize()
+        s.run(8)
+        assert s.launch_count == 1 + 8
+        L.fake.fake_launches(b"", 1)
+        s.adjoint_gradient(8, 8)
+        assert L.fake.fake_launches(b"sweep_kernel", 0) == 0
+
+
+def test_synchronize_always_looks_at_the_error_word(L):
+    """A sweep or pipelined step in a graph captured by the caller may run after
+    the launch's own check."""
+    flags, per, _ = L.geometry("channel", (64, 64, 64), (1, 0, 0))
+    for call in ("synchronize", "run_timed", "time_launches"):
+        with L.Solver(flags, per, "aa", L.F64) as s:
+            s.run(8)
+            s.synchronize()
+            L.fake.fake_raise(1)
+            with pytest.raises(L.LbmError, match="bulk copies"):
+                getattr(s, call)(*(() if call == "synchronize" else (1,)))
+            s.run(9)
+            assert s.launch_count < s.steps_done  # not a sweep's fault: it still sweeps
+
+
+def test_no_sweep_switch(L, monkeypatch):
+    monkeypatch.setenv("LBM_B200_NO_SWEEP", "1")
+    with _porous_solver(L, (64, 64, 64)) as s:
+        s.run(8)
+        assert s.launch_count == 8
+        L.fake.fake_launches(b"", 1)
+        s.adjoint_gradient(8, 8)
+        assert L.fake.fake_launches(b"sweep_kernel", 0) == 0

@@ -62,3 +62,28 @@ def test_wide_offsets(kind):
                 assert s.launch_count == 2
                 out = s.compare(ref)
                 assert out[0] == out[2] == out[4] == 0.0 and out[3] > 0.0
+
+
+@pytest.mark.parametrize("compact", [False, True])
+@pytest.mark.parametrize("precision", [L.F64, L.F32])
+def test_a_wait_that_runs_out_is_reported(monkeypatch, precision, compact):
+    """With no polls allowed, blocks of the second step that run beside the first
+    give up at once: the kernel ends, the call says so, and the solver goes on
+    in single steps from the state it is given next."""
+    flags, per, _ = L.geometry("channel", (20, 20, 40), (1, 0, 0))
+    f0 = L.perturbed_equilibrium(flags, seed=4, amplitude=2e-3)
+    with L.Solver(flags, per, "aa", precision, compact=compact) as s:
+        s.set_state(f0)
+        for _ in range(8):
+            s.run(1)
+        ref = s.get_state()
+    monkeypatch.setenv("LBM_B200_SWEEP_SPIN", "0")
+    with L.Solver(flags, per, "aa", precision, compact=compact) as s:
+        s.set_state(f0)
+        s.run(8)
+        with pytest.raises(L.LbmError, match="gave up waiting"):
+            s.synchronize()
+        s.set_state(f0)
+        s.run(8)
+        assert np.array_equal(s.get_state(), ref)
+        assert s.launch_count == 1 + 8
