@@ -120,7 +120,8 @@ int lbm_set_fp16_scale(lbm_solver *s, double scale);
 
 /* Per-cell porosity phi in [0,1] (float[nx*ny*nz]) and Brinkman scale alpha:
  * every fluid cell's collision adds the resistance force
- * F_b = -alpha (1 - phi) j (j = momentum). alpha = 0 switches it off.
+ * F_b = -alpha (1 - phi) j (j = momentum). alpha = 0 switches it off, and
+ * gives back the memory that lbm_adjoint_gradient keeps.
  * No counterpart in the reference. */
 int lbm_set_porosity(lbm_solver *s, const float *porosity, double alpha);
 
@@ -373,7 +374,11 @@ int lbm_objective(lbm_solver *s, double *j);
  * obstacles); *j_out (may be NULL): J of the final state; info (may be NULL,
  * 6 doubles): forward ms, reverse ms (recomputation + adjoint), interval,
  * checkpoints, extra device bytes, peak device bytes. The solver's state is
- * left at the initial state. No counterpart in the reference. */
+ * left at the initial state. The extra device memory, up to 4 GB of it, stays
+ * with the solver for its next gradient (lbm_device_bytes counts it) until
+ * lbm_set_porosity switches the porosity off, the solver is destroyed, or an
+ * allocation of this library on the device would fail without it. No
+ * counterpart in the reference. */
 #define LBM_CKPT_AUTO (-1)
 int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_every, double *grad,
     double *j_out, double *info);

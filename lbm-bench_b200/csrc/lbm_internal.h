@@ -13,6 +13,11 @@
 #include "lbm_sweep.cuh"
 #include "lbm_step_x2.cuh"
 
+namespace lbm {
+// cudaMalloc that gives idle adjoint workspaces back before it fails (lbm_solver.cu)
+cudaError_t device_malloc(void **p, size_t bytes);
+} // namespace lbm
+
 extern "C" void lbm_map_pages(void *p, size_t bytes); // host/lbm_host.c
 
 namespace lbm {

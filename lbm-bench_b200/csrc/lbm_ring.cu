@@ -327,7 +327,7 @@ extern "C" int lbm_ring_create(lbm_ring **out, lbm_solver *s, int rank, int nran
   int rc = LBM_OK;
   cudaError_t e = cudaSetDevice(r->device);
   if (e == cudaSuccess)
-    e = cudaMalloc(&r->buf, 4 * r->stride);
+    e = device_malloc((void **)&r->buf, 4 * r->stride);
   if (e == cudaSuccess)
     e = cudaMemset(r->buf, 0, 4 * r->stride);
   for (int i = 0; i < 2 && e == cudaSuccess; ++i)

@@ -18,6 +18,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "lbm_b200.h"
@@ -77,7 +78,7 @@ struct lbm_solver {
   int no_quad;    // FP16 AA: never use the four-cell kernels
   void *u_save_next; // adjoint recomputation: momentum output of the next step
   void *adj_ws;      // adjoint workspace kept between gradients, or NULL
-  size_t adj_bytes;
+  size_t adj_bytes;  // its size, not in dev_bytes
   int slab;          // x-slab of a decomposed domain: device planes 0 and nx+1 are ghosts
   int tma;           // FP64 steps use the bulk-copy pipelined kernels (shape in tma_shape)
   int tma_groups;    // consumer groups of 8 warps per CTA
@@ -541,6 +542,56 @@ static int need_device(void)
   return LBM_OK;
 }
 
+// Solvers whose kept adjoint workspace (adj_ws) no gradient is using. Whoever
+// frees or takes one holds the mutex; a gradient in progress is not listed.
+static std::mutex g_idle_mu;
+static std::vector<lbm_solver *> g_idle;
+
+static void drop_workspace(lbm_solver *s)
+{
+  cudaFree(s->adj_ws); // waits for what uses it
+  s->adj_ws = NULL;
+  s->adj_bytes = 0;
+}
+
+// Takes a solver's workspace out of the list: for its own use, or to free it.
+static void take_workspace(lbm_solver *s, bool drop)
+{
+  std::lock_guard<std::mutex> lock(g_idle_mu);
+  g_idle.erase(std::remove(g_idle.begin(), g_idle.end(), s), g_idle.end());
+  if (drop)
+    drop_workspace(s);
+}
+
+// Bytes of the idle workspaces of a device.
+static size_t idle_workspaces(int device)
+{
+  std::lock_guard<std::mutex> lock(g_idle_mu);
+  size_t n = 0;
+  for (const lbm_solver *s : g_idle)
+    n += s->device == device ? s->adj_bytes : 0;
+  return n;
+}
+
+// cudaMalloc that gives idle workspaces of the current device back before it
+// fails.
+cudaError_t lbm::device_malloc(void **p, size_t bytes)
+{
+  cudaError_t e = cudaMalloc(p, bytes);
+  int device = -1;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess)
+    return e;
+  std::lock_guard<std::mutex> lock(g_idle_mu);
+  const auto here = std::stable_partition(g_idle.begin(), g_idle.end(),
+      [&](const lbm_solver *s) { return s->device != device; });
+  if (here == g_idle.end())
+    return e;
+  cudaGetLastError();
+  std::for_each(here, g_idle.end(), drop_workspace);
+  g_idle.erase(here, g_idle.end());
+  return cudaMalloc(p, bytes);
+}
+
 static void free_all(lbm_solver *s)
 {
   if (!s)
@@ -557,7 +608,7 @@ static void free_all(lbm_solver *s)
   cudaFree(s->cwb);
   delete s->cplane0;
   cudaFree(s->sweep_done);
-  cudaFree(s->adj_ws);
+  take_workspace(s, true);
   free(s->split_done);
   if (s->fork_ev)
     cudaEventDestroy(s->fork_ev);
@@ -584,7 +635,7 @@ static void free_all(lbm_solver *s)
 
 static int dev_alloc(lbm_solver *s, void **p, size_t bytes, const char *what)
 {
-  cudaError_t e = cudaMalloc(p, bytes);
+  cudaError_t e = device_malloc(p, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = NULL;
@@ -929,9 +980,9 @@ static int create_impl(lbm_solver **out, int nx, int ny, int nz, const int *flag
   const long long dense_plane = (cells + pq - 1) / pq * pq;
   uint32_t *dmask = s->mask;
   if (s->compact)
-    TRYC(cudaMalloc((void **)&dmask, (size_t)dense_plane * 4));
+    TRYC(device_malloc((void **)&dmask, (size_t)dense_plane * 4));
   uint8_t *dfluid = NULL;
-  cudaError_t e = cudaMalloc((void **)&dfluid, (size_t)cells);
+  cudaError_t e = device_malloc((void **)&dfluid, (size_t)cells);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(dfluid, fluid.data(), (size_t)cells, cudaMemcpyHostToDevice, s->stream);
   if (e == cudaSuccess) {
@@ -1061,6 +1112,7 @@ extern "C" int lbm_set_porosity(lbm_solver *s, const float *porosity, double alp
     return fail(LBM_ERR_ARG, "lbm_set_porosity: NULL solver");
   if (alpha == 0.0) {
     s->alpha = 0.0;
+    take_workspace(s, true); // no gradient without it
     return LBM_OK;
   }
   if (!porosity || !(alpha > 0.0))
@@ -2509,6 +2561,8 @@ __global__ void grad_to_dense_kernel(Grid g, UserBox u, const double *__restrict
 }
 
 // Largest adjoint workspace a solver keeps between gradients: 2% of the device.
+// It is given back when an allocation of this library does not fit, when the
+// porosity is switched off, and with the solver.
 constexpr size_t kKeptWorkspace = (size_t)4 << 30;
 
 // Runs `len` Brinkman steps, saving the momentum of step i at ub + i * ubytes.
@@ -2624,7 +2678,7 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
   if (k == LBM_CKPT_AUTO) {
     size_t free_b = 0, total_b = 0;
     CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    const double budget = 0.9 * (double)(free_b + s->adj_bytes);
+    const double budget = 0.9 * (double)(free_b + idle_workspaces(s->device));
     k = std::min(k_sqrt, steps);
     // memory grows with k beyond k_sqrt; the largest fitting k by bisection
     long long lo = k, hi = steps;
@@ -2659,12 +2713,10 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
   {
     // one workspace, kept for the solver's next gradient when it is small
     // (allocating and freeing it took 3-4 of 20 ms at 96^3 x 100 steps)
-    if (s->adj_bytes < extra) {
-      cudaFree(s->adj_ws);
-      s->adj_ws = NULL;
-      s->dev_bytes -= s->adj_bytes;
-      s->adj_bytes = 0;
+    take_workspace(s, s->adj_bytes < extra);
+    if (!s->adj_ws) {
       RTRY(dev_alloc(s, &s->adj_ws, extra, "the adjoint workspace"));
+      s->dev_bytes -= extra;
       s->adj_bytes = extra;
     }
     dg = (double *)s->adj_ws; // each part is a multiple of the plane's 256 bytes
@@ -2760,16 +2812,16 @@ extern "C" int lbm_adjoint_gradient(lbm_solver *s, int steps, int checkpoint_eve
       info[2] = k;
       info[3] = nck;
       info[4] = (double)extra;
-      info[5] = (double)(s->dev_bytes - s->adj_bytes + extra);
+      info[5] = (double)(s->dev_bytes + extra);
     }
   }
 done:
   s->u_save_next = NULL;
   if (s->adj_bytes > kKeptWorkspace || rc) {
-    cudaFree(s->adj_ws); // waits for what uses it
-    s->adj_ws = NULL;
-    s->dev_bytes -= s->adj_bytes;
-    s->adj_bytes = 0;
+    drop_workspace(s);
+  } else {
+    std::lock_guard<std::mutex> lock(g_idle_mu);
+    g_idle.push_back(s);
   }
   if (e0)
     cudaEventDestroy(e0);
@@ -2798,7 +2850,11 @@ extern "C" int lbm_unpin_host(void *ptr)
 
 extern "C" long long lbm_fluid_cells(const lbm_solver *s) { return s ? s->n_fluid : -1; }
 extern "C" long long lbm_steps_done(const lbm_solver *s) { return s ? s->steps_done : -1; }
-extern "C" size_t lbm_device_bytes(const lbm_solver *s) { return s ? s->dev_bytes : 0; }
+extern "C" size_t lbm_device_bytes(const lbm_solver *s)
+{
+  std::lock_guard<std::mutex> lock(g_idle_mu);
+  return s ? s->dev_bytes + s->adj_bytes : 0;
+}
 extern "C" long long lbm_launch_count(const lbm_solver *s) { return s ? s->launches : -1; }
 extern "C" double lbm_bytes_per_update(const lbm_solver *s)
 {

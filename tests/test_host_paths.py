@@ -51,13 +51,14 @@ def test_failed_staging_growth_leaves_the_solver_usable(L):
     staging the solver was created with: growing it fails, and the gradient's
     download, which needs no more than before, still has its buffer."""
     with _porous_solver(L, (1, 1500, 1500)) as s:
-        s.adjoint_gradient(2, 1)
         before = s.device_bytes
         L.fake.fake_limit(L.fake.fake_used() + (1 << 20))
         with pytest.raises(L.LbmError):
             s.moments()
         L.fake.fake_limit(1 << 40)
+        assert s.device_bytes == before
         s.adjoint_gradient(2, 1)
+        s.set_porosity(np.zeros((1, 1500, 1500), np.float32), 0.0)
         assert s.device_bytes == before
         s.moments()
         assert s.device_bytes > before
@@ -209,3 +210,33 @@ def test_no_sweep_switch(L, monkeypatch):
         L.fake.fake_launches(b"", 1)
         s.adjoint_gradient(8, 8)
         assert L.fake.fake_launches(b"sweep_kernel", 0) == 0
+
+
+def test_kept_adjoint_workspace_is_given_back(L):
+    """A solver keeps its workspace between gradients; a second gradient or a
+    second solver that would not fit without that memory gets it, and switching
+    the porosity off gives it back."""
+    dims = (64, 64, 64)
+    with _porous_solver(L, dims) as a:
+        own = a.device_bytes
+        g = a.adjoint_gradient(30, 30)[2]
+        kept = a.device_bytes - own
+        assert kept == g["extra_bytes"] > 4 * own and g["peak_bytes"] == own + kept
+        try:
+            # room for a second solver, but not for its gradient
+            L.fake.fake_limit(L.fake.fake_used() + own + (8 << 20))
+            with _porous_solver(L, dims) as b:
+                # AUTO: the longest interval, with what a keeps counted as free
+                assert b.adjoint_gradient(9, L.CKPT_AUTO)[2]["interval"] == 9
+                assert a.device_bytes == own < b.device_bytes
+                a.adjoint_gradient(30, 30)  # and the other way round
+                assert b.device_bytes == own and a.device_bytes == own + kept
+                with _porous_solver(L, dims):
+                    assert a.device_bytes == own
+                a.adjoint_gradient(30, 30)
+            assert a.device_bytes == own + kept == L.fake.fake_used()
+        finally:
+            L.fake.fake_limit(1 << 40)
+        a.set_porosity(np.zeros(dims, np.float32), 0.0)
+        assert a.device_bytes == own == L.fake.fake_used()
+    assert L.fake.fake_used() == 0
