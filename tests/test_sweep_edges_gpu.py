@@ -87,3 +87,34 @@ def test_a_wait_that_runs_out_is_reported(monkeypatch, precision, compact):
         s.run(8)
         assert np.array_equal(s.get_state(), ref)
         assert s.launch_count == 1 + 8
+
+
+@pytest.mark.parametrize("dims", [(12, 10, 64), (9, 11, 128), (8, 9, 256)])
+@pytest.mark.parametrize("per", [(1, 0, 0), (1, 1, 1), (0, 1, 1)])
+@pytest.mark.parametrize("precision", [L.F64, L.F32, L.F16])
+def test_rows_of_whole_segments(monkeypatch, precision, per, dims):
+    """For nz a multiple of 64 (128) the single steps of the dense layout run
+    shuffle-aligned (four-cell) kernels: they, the generic two-cell kernels,
+    the compact layout's and the sweeps agree, odd and even steps, with walls."""
+    flags = (np.random.default_rng(sum(dims) + sum(per)).uniform(size=dims[::-1]) > 0.25)
+    flags = flags.astype(np.int32)
+    for axis in range(3):
+        if not per[axis]:
+            face = [slice(None)] * 3
+            face[2 - axis] = [0, -1]
+            flags[tuple(face)] = 0
+    assert flags.sum() >= 4096
+    for pattern in ("aa", "pull", "push"):
+        out = {}
+        for switch in ("", "LBM_B200_NO_SHUFFLE", "LBM_B200_NO_QUAD"):
+            for name in ("LBM_B200_NO_SHUFFLE", "LBM_B200_NO_QUAD"):
+                monkeypatch.setenv(name, "1" if name == switch else "0")
+            out[switch or "aligned"], = _states(flags, per, pattern, precision, False, ((1,) * 7,))
+        out["compact"], = _states(flags, per, pattern, precision, True, ((1,) * 7,))
+        assert all(launches == 7 for _, launches in out.values())
+        for compact in (False, True):
+            out["sweep", compact], = _states(flags, per, pattern, precision, compact, ((7,),))
+            assert out["sweep", compact][1] == 2
+        ref = out["aligned"][0]
+        for name, (state, _) in out.items():
+            assert np.array_equal(state, ref), (pattern, name)
