@@ -118,3 +118,31 @@ def test_rows_of_whole_segments(monkeypatch, precision, per, dims):
         ref = out["aligned"][0]
         for name, (state, _) in out.items():
             assert np.array_equal(state, ref), (pattern, name)
+
+
+@pytest.mark.parametrize("per", [(1, 1, 1), (1, 1, 0)])
+@pytest.mark.parametrize("precision,dims,compact,patterns", [
+    (L.F16, (8, 600, 600), False, ("aa", "push", "pull")),
+    (L.F16, (8, 600, 600), True, ("push", "pull")),  # AA keeps single steps there
+    (L.F32, (8, 500, 431), False, ("aa", "push", "pull")),
+    (L.F32, (8, 500, 431), True, ("aa", "push", "pull"))])
+def test_fronts_in_two_slabs(precision, dims, compact, patterns, per):
+    """Planes of more than 9 MB: two y slabs, whose rows the second step shifts
+    by one; two cells of a pair can belong to different slabs."""
+    flags = (np.random.default_rng(7).uniform(size=dims[::-1]) > 0.05).astype(np.int32)
+    for pattern in patterns:
+        (ref, singles), (got, launches) = _states(flags, per, pattern, precision, compact,
+                                                  ((1,) * 4, (4,)))
+        assert singles == 4 and launches == 2
+        assert np.array_equal(got, ref), pattern
+
+
+@pytest.mark.parametrize("pattern", ["aa", "push"])
+@pytest.mark.parametrize("dims,launches", [((24, 30, 41), 1), ((70, 221, 203), 3)])
+def test_fp16_brinkman_sweeps(dims, launches, pattern):
+    flags, _, _ = L.porous_channel(dims, 0.25, 2.0, 5.0, seed=3)
+    por = np.random.default_rng(4).uniform(0, 1, dims).astype(np.float32)
+    (ref, singles), (got, n) = _states(flags, (1, 0, 0), pattern, L.F16, False,
+                                       ((1,) * 6, (6,)), porosity=por)
+    assert singles == 6 and n == launches
+    assert np.array_equal(got, ref)
