@@ -100,6 +100,7 @@ struct lbm_solver {
   // sweeps (lbm_sweep.cuh): several steps per launch, planned at creation
   int no_sweep;         // LBM_B200_NO_SWEEP=1, or a sweep's wait ran out: single steps only
   int sweep_steps;      // most steps of one launch; 0: single steps only
+  int sweep_least;      // fewer steps than this run as single ones
   SweepPlan sweep;
   uint32_t *sweep_done; // its counters
   int err_pending;      // a launch that may set dev_err is not yet checked
@@ -742,6 +743,7 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
   if (const char *spin = getenv("LBM_B200_SWEEP_SPIN")) // polls before a wait gives up
     s->sweep.spin = (uint32_t)strtoul(spin, NULL, 10);
   s->sweep_steps = steps;
+  s->sweep_least = sweep_least(u, fronts);
   return LBM_OK;
 }
 
@@ -1946,7 +1948,8 @@ static int next_sweep(const lbm_solver *s, int left)
     return 0;
   if (s->pattern == LBM_PULL && s->alpha != 0.0 && s->porosity)
     return 0; // no Brinkman term in the pull orientation
-  return std::min(left & ~1, s->sweep_steps);
+  const int n = std::min(left & ~1, s->sweep_steps);
+  return n >= s->sweep_least ? n : 0;
 }
 
 extern "C" int lbm_run(lbm_solver *s, int steps)

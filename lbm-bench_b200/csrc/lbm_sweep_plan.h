@@ -290,4 +290,20 @@ inline bool sweep_pays(const SweepUse &u, bool fronts)
   return u.fill >= (u.zper ? 0.03 : 0.015) && !(u.nz % 128 == 0 && u.fluid > 0.9);
 }
 
+// Steps from which a sweep pays: a step-major launch of two steps still has the
+// clearing of its counters and one full wait for two launches. Calls of lbm_run
+// back to back, us a step, single steps / sweep, channels: 20^3 FP64 AA dense 4.1
+// / 5.0 in calls of two steps, 4.1 / 3.7 of four; 32^3 FP32 push compact 4.2 / 5.2,
+// 4.1 / 4.1; 200 x 64^2 FP16 AA compact 16.8 / 19.1; but 64^3 FP64 push dense
+// 12.7 / 11.8, 20^3 FP32 push dense 6.2 / 5.2, periodic 20^2 x 40 FP16 pull
+// compact 10.3 / 5.2.
+inline int sweep_least(const SweepUse &u, bool fronts)
+{
+  if (fronts || (u.compact && u.zper))
+    return 2;
+  if (u.bytes == 2 && (u.compact ? u.aa : u.pull))
+    return 4;
+  return u.waves < 0.5 && (u.compact || u.pull || u.bytes == 8) ? 4 : 2;
+}
+
 } // namespace lbm

@@ -240,3 +240,20 @@ def test_kept_adjoint_workspace_is_given_back(L):
         a.set_porosity(np.zeros(dims, np.float32), 0.0)
         assert a.device_bytes == own == L.fake.fake_used()
     assert L.fake.fake_used() == 0
+
+
+@pytest.mark.parametrize("dims,kind,pattern,precision,compact,least", [
+    ((20, 20, 20), "channel", "aa", "fp64", False, 4),
+    ((32, 32, 32), "channel", "push", "fp32", True, 4),
+    ((200, 64, 64), "channel", "aa", "fp16", True, 4),
+    ((64, 64, 64), "channel", "push", "fp64", False, 2),
+    ((20, 20, 40), "fluid", "pull", "fp16", True, 2),
+    ((128, 128, 128), "channel", "aa", "fp64", True, 2)])
+def test_short_calls(L, dims, kind, pattern, precision, compact, least):
+    """Calls of two or three steps sweep where that is faster."""
+    flags, per, _ = L.geometry(kind, dims, (1, 0, 0))
+    with L.Solver(flags, per, L.PATTERNS[pattern], L.PRECISIONS[precision], compact=compact) as s:
+        s.run(2)
+        assert s.launch_count == (1 if least == 2 else 2)
+        s.run(least)
+        assert s.launch_count == (2 if least == 2 else 3)
