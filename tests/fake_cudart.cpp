@@ -14,6 +14,7 @@
 namespace {
 std::map<char *, size_t> g_live;
 size_t g_limit = (size_t)1 << 40, g_used = 0;
+long g_mapped = 0; // allocations of 1 MB and more: each maps device memory of its own
 std::map<const void *, std::string> g_names;
 std::map<std::string, long> g_count;
 cudaError_t g_last = cudaSuccess;
@@ -62,6 +63,7 @@ cudaError_t clear(void *p, int v, size_t n)
 extern "C" {
 void fake_limit(size_t bytes) { g_limit = bytes; }
 size_t fake_used(void) { return g_used; }
+long fake_mapped(void) { return g_mapped; }
 // launches since the last reset of kernels whose mangled name contains `part`
 long fake_launches(const char *part, int reset)
 {
@@ -119,6 +121,7 @@ cudaError_t cudaMalloc(void **p, size_t n)
   *p = std::calloc(1, n ? n : 1);
   g_live[(char *)*p] = n;
   g_used += n;
+  g_mapped += n >= (size_t)1 << 20;
   return cudaSuccess;
 }
 cudaError_t cudaFree(void *p)

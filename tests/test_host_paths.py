@@ -35,6 +35,7 @@ def L(tmp_path_factory):
     mod.fake.fake_limit.argtypes = [ctypes.c_size_t]
     mod.fake.fake_used.restype = ctypes.c_size_t
     mod.fake.fake_launches.restype = ctypes.c_long
+    mod.fake.fake_mapped.restype = ctypes.c_long
     yield mod
     mod.fake.fake_limit(1 << 40)
 
@@ -64,13 +65,28 @@ def test_failed_staging_growth_leaves_the_solver_usable(L):
         assert s.device_bytes > before
 
 
+@pytest.mark.parametrize("pattern,lattices", [("aa", 1), ("push", 2)])
 @pytest.mark.parametrize("compact", [False, True])
-def test_creation_needs_no_memory_for_what_it_can_do_without(L, compact):
+def test_creation_maps_memory_for_the_lattices_only(L, compact, pattern, lattices):
+    """A small solver's other buffers come out of memory that is mapped anyway."""
+    flags, per, _ = L.geometry("box", (20, 20, 20))
+    before = L.fake.fake_mapped()
+    with L.Solver(flags, per, L.PATTERNS[pattern], L.F64, compact=compact) as s:
+        s.set_state(np.zeros((19, 20, 20, 20)))
+        s.run(8)
+        s.get_state()
+        s.moments()
+        assert L.fake.fake_mapped() - before <= lattices
+    assert L.fake.fake_used() == 0
+
+
+@pytest.mark.parametrize("dims", [(512, 16, 32), (128, 32, 32)])
+@pytest.mark.parametrize("compact", [False, True])
+def test_creation_needs_no_memory_for_what_it_can_do_without(L, compact, dims):
     """On a nearly full device a solver is created without the sweeps'
     counters and with staging for one dense plane, and takes single steps."""
-    dims = (512, 16, 32)
     flags = np.ones(dims[::-1], np.int32)
-    cells = 512 * 16 * 32
+    cells = dims[0] * dims[1] * dims[2]
 
     def make():
         return L.Solver(flags, (1, 1, 1), "aa", L.F64, compact=compact)
@@ -92,7 +108,7 @@ def test_creation_needs_no_memory_for_what_it_can_do_without(L, compact):
             with make() as s:
                 s.run(8)
                 assert s.steps_done == 8
-                assert s.launch_count == 8 or limit > least
+                assert s.launch_count == 8 or limit > least or dims[0] == 128
                 s.get_state()
                 s.moments()
     finally:
