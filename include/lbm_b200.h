@@ -281,8 +281,12 @@ int lbm_device_memory(size_t *free_bytes, size_t *total_bytes);
  * steps may run in one launch; the states are those of single steps, bit for
  * bit.
  * Replaces the time loop of kd->Kernel (src/kernel_pull_soa.c:44-214,
- * src/kernel_push_soa.c:44-214, src/kernel_aa_soa.c:36-286); an AA solver
- * runs single steps, so odd counts are allowed. */
+ * src/kernel_push_soa.c:44-214, src/kernel_aa_soa.c:36-286). Any count is
+ * allowed in every pattern: where launches take pairs of steps, an odd step
+ * runs by itself. A launch that waits for an earlier step of its own gives up
+ * after about a second (never seen outside a test): the next call that waits
+ * reports LBM_ERR_CUDA, the state is undefined until it is set again, and the
+ * solver takes single steps from then on. */
 int lbm_run(lbm_solver *s, int steps);
 int lbm_synchronize(lbm_solver *s);
 

@@ -18,7 +18,7 @@ namespace lbm {
 cudaError_t device_malloc(void **p, size_t bytes);
 } // namespace lbm
 
-extern "C" void lbm_map_pages(void *p, size_t bytes); // host/lbm_host.c
+extern "C" void lbm_map_pages(void *p, size_t bytes); // host/lbm_host.c, not exported
 
 namespace lbm {
 

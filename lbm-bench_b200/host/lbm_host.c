@@ -3,7 +3,6 @@
 #include <math.h>
 #include <stdint.h>
 #include <sys/mman.h>
-#include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
 #include <strings.h>
@@ -225,7 +224,7 @@ int lbm_perturbed_equilibrium(int nx, int ny, int nz, const int *flags, unsigned
  * GPU still works on the steps queued before the download: moments of 128^3
  * (67 MB) 14.4 -> 10.4 ms on an idle GPU, 100 steps and moments 18.0 -> 11.9.
  * On eight threads the idle figure is 7.7, the one behind the steps 12.3. */
-void lbm_map_pages(void *p, size_t bytes)
+__attribute__((visibility("hidden"))) void lbm_map_pages(void *p, size_t bytes)
 {
   const size_t page = 4096;
   const uintptr_t lo = (uintptr_t)p / page * page, hi = (uintptr_t)p + bytes;
