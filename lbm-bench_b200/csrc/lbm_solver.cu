@@ -85,6 +85,7 @@ struct lbm_solver {
   int tma_groups;    // consumer groups of 8 warps per CTA
   TmaShape tma_shape;
   unsigned int *dev_err; // set by kernels whose bounded waits ran out (kErr bits)
+  unsigned int err_clear; // its value without an error
   uint8_t *bc_marks;     // [2][ny][nz]: inlet / outlet cells of the pressure boundary, or NULL
   int bc_on;
   double rho_in, rho_out;
@@ -666,13 +667,14 @@ static int sync_and_check(lbm_solver *s, bool always = false)
     CUDA_TRY(cudaMemcpyAsync(&err, s->dev_err, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
   CUDA_TRY(cudaStreamSynchronize(s->stream));
   s->err_pending = 0;
-  if (!err)
+  if (!(err & kErrBits))
     return LBM_OK;
   if (err & kErrSweepWait) {
     s->no_sweep = 1;
     s->sweep_steps = 0;
   }
-  CUDA_TRY(cudaMemsetAsync(s->dev_err, 0, sizeof(err), s->stream));
+  CUDA_TRY(cudaMemcpyAsync(s->dev_err, &s->err_clear, sizeof(err), cudaMemcpyHostToDevice,
+      s->stream));
   return fail(LBM_ERR_CUDA, "a step kernel gave up waiting for %s; the state is undefined",
       err & kErrBulkCopy ? "its bulk copies" : "the blocks of an earlier step");
 }
@@ -746,8 +748,6 @@ static int init_sweep(lbm_solver *s, const std::vector<uint32_t> &row_start)
     return rc == LBM_ERR_ALLOC ? LBM_OK : rc;
   s->sweep.done = s->sweep_done;
   s->sweep.err = s->dev_err;
-  if (const char *spin = getenv("LBM_B200_SWEEP_SPIN")) // polls before a wait gives up
-    s->sweep.spin = (uint32_t)strtoul(spin, NULL, 10);
   s->sweep_steps = steps;
   s->sweep_least = sweep_least(u, fronts);
   return LBM_OK;
@@ -936,7 +936,11 @@ static int create_once(lbm_solver **out, int nx, int ny, int nz, const int *flag
     TRYC(cudaMemsetAsync(s->buf[1], 0, s->state_bytes, s->stream));
 
   TRY(dev_alloc(s, (void **)&s->dev_err, sizeof(unsigned int), "the kernel error word"));
-  TRYC(cudaMemsetAsync(s->dev_err, 0, sizeof(unsigned int), s->stream));
+  if (const char *spin = getenv("LBM_B200_SWEEP_SPIN")) // polls before a wait gives up
+    s->err_clear = kSweepSpin - (unsigned)std::min<unsigned long>(kSweepSpin,
+        strtoul(spin, NULL, 10));
+  TRYC(cudaMemcpyAsync(s->dev_err, &s->err_clear, sizeof(unsigned int), cudaMemcpyHostToDevice,
+      s->stream));
   {
     // pipelined FP64 kernels (lbm_step_tma.cuh): with LBM_B200_TMA=1;
     // LBM_B200_TMA_T / _STAGES / _GROUPS set the tile rows, pipeline depth

@@ -42,9 +42,11 @@ namespace lbm {
 
 constexpr int kStepThreads = 128;
 
-// Bits of a solver's kernel error word.
-constexpr unsigned kErrBulkCopy = 1u;  // a pipelined step's bulk copy did not arrive
-constexpr unsigned kErrSweepWait = 2u; // a sweep's wait for an earlier step ran out
+// Bits of a solver's kernel error word. The bits below them (0 but in tests)
+// are polls that a sweep's waits count as made when they begin.
+constexpr unsigned kErrBulkCopy = 1u << 30;  // a pipelined step's bulk copy did not arrive
+constexpr unsigned kErrSweepWait = 1u << 31; // a sweep's wait for an earlier step ran out
+constexpr unsigned kErrBits = kErrBulkCopy | kErrSweepWait;
 
 template <class ST> struct StepArgs {
   using S = typename ST::S;

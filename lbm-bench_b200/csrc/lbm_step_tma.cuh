@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(tma_threads(GROUPS), 1) step_kernel_tma(TmaArg
       if (k >= a.stages &&
           !mbar_wait(smem_addr(&empty[s]), (uint32_t)(((k / a.stages) - 1) & 1))) {
         if (lane == 0)
-          atomicOr(a.err, 1u);
+          atomicOr(a.err, kErrBulkCopy);
         break;
       }
       if (lane <= Q)
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(tma_threads(GROUPS), 1) step_kernel_tma(TmaArg
     const int s = k % a.stages;
     if (!mbar_wait(smem_addr(&full[s]), (uint32_t)((k / a.stages) & 1))) {
       if (lane == 0)
-        atomicOr(a.err, 1u);
+        atomicOr(a.err, kErrBulkCopy);
       return;
     }
     const S *pops = reinterpret_cast<const S *>(smem + (size_t)s * a.stage_bytes);

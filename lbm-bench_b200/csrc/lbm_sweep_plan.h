@@ -21,8 +21,7 @@ constexpr uint32_t kSweepSpin = 1u << 20;  // polls of one wait (about a second)
 
 struct SweepPlan {
   uint32_t *done = nullptr;     // [steps - 1][slabs][nx] counters, kSweepPad words apart
-  unsigned int *err = nullptr;  // set when a wait runs out
-  uint32_t spin = kSweepSpin;   // polls after which it does
+  unsigned int *err = nullptr;  // the solver's error word
   uint32_t nb[2] = { 0, 0 };    // blocks of a plane (and slab) in even / odd steps
   uint32_t front = 0;           // nb[0] + nb[1]
   uint32_t slab_blocks = 0;     // fronts: blocks of a slab

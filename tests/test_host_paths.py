@@ -33,6 +33,7 @@ def L(tmp_path_factory):
     mod.LIB_PATH = str(so)
     mod.fake = mod.lib()
     mod.fake.fake_limit.argtypes = [ctypes.c_size_t]
+    mod.fake.fake_raise.argtypes = [ctypes.c_uint]
     mod.fake.fake_used.restype = ctypes.c_size_t
     mod.fake.fake_launches.restype = ctypes.c_long
     mod.fake.fake_mapped.restype = ctypes.c_long
@@ -192,7 +193,7 @@ def test_a_sweep_that_gave_up_leaves_single_steps(L):
     with _porous_solver(L, (64, 64, 64)) as s:
         s.run(8)
         assert s.launch_count == 1
-        L.fake.fake_raise(2)
+        L.fake.fake_raise(1 << 31)
         with pytest.raises(L.LbmError, match="gave up waiting"):
             s.synchronize()
         s.synchronize()
@@ -211,7 +212,7 @@ def test_synchronize_always_looks_at_the_error_word(L):
         with L.Solver(flags, per, "aa", L.F64) as s:
             s.run(8)
             s.synchronize()
-            L.fake.fake_raise(1)
+            L.fake.fake_raise(1 << 30)
             with pytest.raises(L.LbmError, match="bulk copies"):
                 getattr(s, call)(*(() if call == "synchronize" else (1,)))
             s.run(9)

@@ -67,9 +67,9 @@ def test_wide_offsets(kind):
 @pytest.mark.parametrize("compact", [False, True])
 @pytest.mark.parametrize("precision", [L.F64, L.F32])
 def test_a_wait_that_runs_out_is_reported(monkeypatch, precision, compact):
-    """With no polls allowed, blocks of the second step that run beside the first
-    give up at once: the kernel ends, the call says so, and the solver goes on
-    in single steps from the state it is given next."""
+    """With no polls allowed, blocks of later steps that run beside the first give
+    up at their sixteenth: the kernel ends, the call says so, and the solver goes
+    on in single steps from the state it is given next."""
     flags, per, _ = L.geometry("channel", (20, 20, 40), (1, 0, 0))
     f0 = L.perturbed_equilibrium(flags, seed=4, amplitude=2e-3)
     with L.Solver(flags, per, "aa", precision, compact=compact) as s:
