@@ -81,14 +81,22 @@ def measured_hbm_peak():
 
 
 def ncu_traffic(kind: str, precision: str):
-    """DRAM bytes per fluid cell update of `kind` from the committed ncu
-    summary (profiles/traffic.json), or None."""
+    """DRAM bytes per fluid cell of one launch of `kind` (a step, or a sweep of
+    two) from the committed ncu summary (profiles/traffic.json), or None."""
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as fh:
             t = json.load(fh)
-        return float(t[precision][kind]["dram_bytes_per_fluid_update"])
+        per = "cell_and_launch" if kind == "sweep" else "update"
+        return float(t[precision][kind][f"dram_bytes_per_fluid_{per}"])
     except Exception:
         return None
+
+
+def hbm_gbs(s, launches_before: int, ms: float) -> float:
+    """GB/s of the populations through HBM: one read and one write per launch
+    since `launches_before`, for one step or (a sweep) for two."""
+    launches = s.launch_count - launches_before
+    return s.fluid_cells * s.bytes_per_update * launches / (ms / 1e3) / 1e9
 
 
 class ClockSampler:
@@ -282,10 +290,8 @@ def run_native(args, dist: Dist):
     flags, f0, frac, nsph = make_workload(L, n)
     peak, peak_kind = measured_hbm_peak()
 
-    # ---- headline: FP64 AA, device-resident, lbm_run between CUDA events. Its sweeps
-    # take a plane's populations through HBM once per two steps, so the figures in
-    # bytes per update and second below can pass the copy peak; the roofline is that
-    # of the single-step kernels
+    # ---- headline: FP64 AA, device-resident, lbm_run between CUDA events. A launch
+    # reads and writes the populations once, for one step or (a sweep) for two
     compact = args.layout == "compact"
     other = "dense" if compact else "compact"
     s = solver(L, flags, "aa", L.F64, f0, compact)
@@ -301,22 +307,31 @@ def run_native(args, dist: Dist):
         s.synchronize()
     dist.barrier()
     launches = s.launch_count - launches0
-    # the single-step kernels one by one, for the roofline
+    # the single-step kernels one by one, which slabs and odd steps use
     per_kind, _ = s.time_launches(args.steps)
     ms = dist.max(region_ms)
     tot, bad = s.mass_momentum(check=False)
     value = dist.world * n_fluid * args.steps / (ms / 1e3) / 1e6
-    dom = max(per_kind, key=lambda k: per_kind[k][0])
-    dom_ms = per_kind[dom][0] / per_kind[dom][1]
-    achieved = n_fluid * bpu / (dom_ms / 1e3) / 1e9
-    traffic = ncu_traffic(dom, "fp64_compact" if compact else "fp64")
-    kname = (("step_kernel_cp_local<StoreF64>" if dom == "aa_even" else
-              f"step_kernel_cp<StoreF64,{dom}>") if compact else f"step_kernel<StoreF64,{dom}>")
-    roofline = {"bound": "hbm", "kernel": kname, "layout": args.layout, "achieved": achieved,
+    prec_key = "fp64_compact" if compact else "fp64"
+
+    def of_peak(kernel, kind, launch_ms):
+        achieved = n_fluid * bpu / (launch_ms / 1e3) / 1e9
+        traffic = ncu_traffic(kind, prec_key)
+        return {"bound": "hbm", "kernel": kernel, "layout": args.layout, "achieved": achieved,
                 "peak": peak, "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic * n_fluid if traffic else None,
-                "algorithmic_bytes_per_launch": n_fluid * bpu,
-                "launch_ms": dom_ms, "per_kind_ms": {k: v[0] / v[1] for k, v in per_kind.items()}}
+                "algorithmic_bytes_per_launch": n_fluid * bpu, "launch_ms": launch_ms}
+
+    dom = max(per_kind, key=lambda k: per_kind[k][0])
+    single = of_peak((("step_kernel_cp_local<StoreF64>" if dom == "aa_even" else
+                       f"step_kernel_cp<StoreF64,{dom}>") if compact else
+                      f"step_kernel<StoreF64,{dom}>"), dom, per_kind[dom][0] / per_kind[dom][1])
+    single["per_kind_ms"] = {k: v[0] / v[1] for k, v in per_kind.items()}
+    roofline = single
+    if launches < args.steps:
+        roofline = of_peak(f"sweep_kernel<Sweep{'Cp' if compact else 'Dense'}<StoreF64>>", "sweep",
+                           region_ms / launches)
+        roofline["steps_per_launch"] = args.steps / launches
 
     # ---- variants (same workload): FP64 pull/push, FP32/FP16 AA with error vs FP64
     variants = {}
@@ -327,11 +342,12 @@ def run_native(args, dist: Dist):
                         ("pull", not compact), ("push", not compact)):
         v = solver(L, flags, pattern, L.F64, f0, cp)
         v.run(args.warmup)
+        before = v.launch_count
         t = v.run_timed(vsteps)
         key = f"fp64_{pattern}" + ("" if cp == compact else f"_{other}")
         variants[key] = {
             "mlups": n_fluid * vsteps / (t / 1e3) / 1e6,
-            "gbs": n_fluid * vsteps * v.bytes_per_update / (t / 1e3) / 1e9,
+            "gbs": hbm_gbs(v, before, t),
             "layout": "compact" if cp else "dense", "device_bytes": v.device_bytes}
         variants[key]["frac"] = variants[key]["gbs"] / peak
         v.close()
@@ -342,12 +358,14 @@ def run_native(args, dist: Dist):
         for pattern, cp in (("aa", False), ("pull", False), ("aa", True), ("pull", True)):
             b = solver(L, flags, pattern, prec, f0, cp)
             b.run(args.warmup)
+            before = b.launch_count
             t = b.run_timed(args.steps - args.warmup) if args.steps > args.warmup else None
+            gbs = hbm_gbs(b, before, t) if t else None
             d = b.compare(ref)
             mlups = n_fluid * (args.steps - args.warmup) / (t / 1e3) / 1e6 if t else None
             key = f"{name}_{pattern}" + ("_compact" if cp else "")
             variants[key] = {
-                "mlups": mlups, "gbs": mlups * b.bytes_per_update / 1e3 if mlups else None,
+                "mlups": mlups, "gbs": gbs,
                 "l2_rel_err_u": float(np.sqrt(d[0] / d[1])) if d[1] > 0 else None,
                 "l2_rel_err_rho": float(np.sqrt(d[2] / d[3])) if d[3] > 0 else None,
                 "error_after_steps": args.steps, "layout": "compact" if cp else "dense"}
@@ -369,8 +387,8 @@ def run_native(args, dist: Dist):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
         "data": "synthetic (seeded porous geometry and initial state)",
         "config": workload_config(n, frac, nsph, n_fluid),
-        "gbs": n_fluid * bpu * args.steps / (ms / 1e3) / 1e9,
-        "roofline": roofline, "e2e": e2e, "gpu_launches": launches,
+        "gbs": n_fluid * bpu * launches / (ms / 1e3) / 1e9,
+        "roofline": roofline, "roofline_single_step": single, "e2e": e2e, "gpu_launches": launches,
         "clocks": clk.summary(), "variants": variants, "adjoint": adjoint,
         "state_check": {"mass": tot[0], "nonfinite_cells": bad},
         "device_bytes": s.device_bytes,
@@ -410,8 +428,8 @@ def summary(r):
     roofline fraction per precision and pattern, errors against FP64, the
     adjoint's cost, and the parity of configs 0 and 1 with the reference."""
     v = r.get("variants", {})
-    out = {"fp64_aa": {"mlups": _r(r["value"]), "frac_step": _r(r["gbs"] / r["roofline"]["peak"]),
-                       "frac_dominant": _r(r["roofline"]["frac"]),
+    out = {"fp64_aa": {"mlups": _r(r["value"]), "frac": _r(r["roofline"]["frac"]),
+                       "frac_single_step": _r(r["roofline_single_step"]["frac"]),
                        "layout": r["roofline"].get("layout")}}
     for k in ("fp64_pull", "fp64_push", "fp64_aa_dense", "fp64_pull_dense", "fp64_push_dense",
               "fp64_aa_compact", "fp64_pull_compact", "fp64_push_compact"):
@@ -662,11 +680,12 @@ def timed_forward(L, flags, pattern, precision, steps, warmup, peak, compact=Fal
     s.set_params(1.25, 3 / 16, 1e-6, True)
     s.init_equilibrium(seed=7, amplitude=1e-4)
     s.run(warmup)
+    before = s.launch_count
     with ClockSampler(0) as clk:
         ms = s.run_timed(steps)
     n_fluid = s.fluid_cells
     mlups = n_fluid * steps / (ms / 1e3) / 1e6
-    gbs = mlups * s.bytes_per_update / 1e3
+    gbs = hbm_gbs(s, before, ms)
     return s, {"mlups": mlups, "gbs": gbs, "frac": gbs / peak, "ms_per_step": ms / steps,
                "fluid_cells": n_fluid, "device_bytes": s.device_bytes,
                "bytes_per_update": s.bytes_per_update, "clocks": clk.summary(),
