@@ -42,6 +42,16 @@ template <typename V> struct AdjArgs {
   V oE, oO, w0, w1, w2, alpha;
 };
 
+// a * b + c. In FP64 rounded once by its own word: the FP64 kernels are compiled
+// without contraction, so that steps and sweeps agree bit for bit, which had made
+// single reverse steps 10-15% slower. 60 steps with their recomputation, ms,
+// contracted / not / with these: 60000 x 5 x 5 26.5 / 30.6 / 27.9, pipe in 200 x
+// 100 x 33 1.92 / 2.11 / 2.00. (The sums of `pair` as well: 27.3 and 1.99, but
+// sweeps spill 120 bytes for 80: 128^3 17.5 for 17.3.) FP32 leaves it to the
+// compiler.
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return a * b + c; }
+
 // One cell's reverse step: mu and the momentum u of the step to lambda^t
 // (store(k, value)) and this step's dJ/dphi (returned).
 template <typename V, class STORE>
@@ -75,12 +85,12 @@ __device__ __forceinline__ V adjoint_cell(const AdjArgs<V> &a, const V (&mu)[Q],
   pair(dTE, dBW, a.w2);
   pair(dTS, dBN, a.w2);
   pair(dTN, dBS, a.w2);
-  gx -= V(3) * ux * sD;
-  gy -= V(3) * uy * sD;
-  gz -= V(3) * uz * sD;
+  gx = mul_add(V(-3) * ux, sD, gx);
+  gy = mul_add(V(-3) * uy, sD, gy);
+  gz = mul_add(V(-3) * uz, sD, gz);
 #pragma unroll
   for (int k = 0; k < Q; ++k) {
-    const V part = (k == dC) ? (V(1) - oE) * mu[dC] : cdir * mu[k] + ccross * mu[inv(k)];
+    const V part = (k == dC) ? (V(1) - oE) * mu[dC] : mul_add(cdir, mu[k], ccross * mu[inv(k)]);
     store(k, part + sD + gx * V(cx(k)) + gy * V(cy(k)) + gz * V(cz(k)));
   }
   return gphi;
@@ -147,6 +157,7 @@ template <typename V> struct SweepAdjArgs : AdjArgs<V> {
   SweepPlan p;
 };
 
+// 80 registers (figures at plan_adjoint_sweep)
 #ifndef LBM_MINB_SWEEP_ADJ
 #define LBM_MINB_SWEEP_ADJ 6
 #endif

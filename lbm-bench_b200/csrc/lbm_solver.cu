@@ -2642,16 +2642,16 @@ static AdjArgs<V> adj_args(const lbm_solver *s, const void *from, void *to, cons
 // first; plan.steps = 0 for single steps. 60 steps' reverse sweep with its
 // recomputation, single / sweep, ms: channels 64^3 (40 MB) 1.65 / 1.13, 96 x
 // 64^2 (60 MB) 2.67 / 1.76 step-major, 128 x 64^2 (80 MB) 3.75 / 2.81, 160^3
-// 25.9 / 18.8 in fronts. Below a third of a block's cells in use, or in a
-// mostly solid box, empty blocks cost more than HBM (16384 x 6^2, 0.06: 11.1 /
-// 12.1; pipe in 300 x 300 x 16: 2.22 / 4.70; 300^2 x 16, 0.43: 12.8 / 10.9).
+// 25.9 / 18.8 in fronts; 300^2 x 8 (a fill of 0.19) 10.2 / 9.8. With fewer of a
+// block's cells in use, or in a mostly solid box, empty blocks cost more than HBM
+// (16384 x 6^2, 0.06: 11.1 / 12.1; pipe in 300 x 300 x 16: 2.22 / 4.70). Blocks
+// per SM: 128^3, 100 steps, 6 17.5, 5 17.8, 4 18.3, 7 19.0.
 static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
 {
   SweepPlan p;
   p.steps = 0;
   if (s->no_sweep || s->precision != LBM_F64 || s->slab || s->tma || s->compact ||
-      s->n_fluid < 4096 ||
-      s->g.nx < 4 || sm_count() == 0 ||
+      s->n_fluid < 4096 || sm_count() == 0 ||
       (unsigned long long)Q * (unsigned long long)s->g.plane >= (1ull << 32))
     return p;
   SweepShape h;
@@ -2667,7 +2667,8 @@ static SweepPlan plan_adjoint_sweep(const lbm_solver *s)
   const bool ok = sweep_plan(h, fronts, p);
   const SweepUse u = sweep_use(h, p, (double)s->n_fluid);
   const double fluid = (double)s->n_fluid / ((double)s->g.nx * s->g.ny * s->g.nz);
-  if (!ok || (u.waves > 3.1 && (u.fill < 0.33 || (fronts && fluid < 0.25))))
+  if (!ok || (fronts && s->g.nx < 4) ||
+      (u.waves > 3.1 && (u.fill < 0.17 || (fronts && fluid < 0.25))))
     p.steps = 0;
   else
     p.steps = fronts ? 2 : kSweepMaxSteps;
